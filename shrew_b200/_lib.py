@@ -71,6 +71,7 @@ class QuantItem(ctypes.Structure):
 
 
 _lib = None
+_host = None
 
 
 class ShrewError(RuntimeError):
@@ -96,6 +97,23 @@ def lib() -> ctypes.CDLL:
             fn.argtypes = args
         _lib = L
     return _lib
+
+
+def host():
+    """The compiled per-call host path (csrc/host_path.cpp), bound to the loaded library's entry points."""
+    global _host
+    if _host is None:
+        try:
+            from . import _host as ext
+        except ImportError as e:
+            raise ImportError("shrew_b200/_host.so is missing or does not load: build it with `python -m shrew_b200.build` "
+                              "(there is no Python fallback for this path)") from e
+        from .quantize import Device
+        L = lib()
+        ext.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in SIGNATURES}, ShrewError,
+                 lambda index: Device.get(f"cuda:{index}").handle.value)
+        _host = ext
+    return _host
 
 
 def check(rc: int, ctx=None) -> None:

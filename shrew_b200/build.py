@@ -1,20 +1,23 @@
-"""Builds libshrewq.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds libshrewq.so (the C-ABI library) in-tree with nvcc for sm_100a, and _host.so (the per-call host path of the
+Python mirror, a CPython extension) with the host compiler.
 
     python -m shrew_b200.build [--force] [--verbose] [--trace]
 
-nvcc cross-compiles without a GPU.  The shared object lands beside this file so that it
-travels with the source tree; nothing is written outside the package directory.
+nvcc cross-compiles without a GPU.  The shared objects land beside this file so that they
+travel with the source tree; nothing is written outside the package directory.
 """
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libshrewq.so")
+HOST_EXT = os.path.join(HERE, "_host.so")
 SOURCES = ["api.cu", "quantize.cu", "quantize_batch.cu", "quantize_modes.cu", "gemv.cu", "gemv_mma.cu", "gemm_simt.cu", "gemm_tcgen05.cu", "gemm_tcgen05_2cta.cu", "exchange.cu"]
 HEADERS = sorted(os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith(".cuh")) + [os.path.join(HERE, "..", "include", "shrewq.h")]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
@@ -35,7 +38,9 @@ def build_library(force: bool = False, verbose: bool = False, trace: bool = Fals
     if trace:
         return _build(os.path.join(CSRC, "build_trace"), os.path.join(HERE, "libshrewq_trace.so"),
                       FLAGS + ["-DSHREWQ_TRACE"], force, verbose)
-    return _build(os.path.join(CSRC, "build"), LIB, FLAGS, force, verbose)
+    lib = _build(os.path.join(CSRC, "build"), LIB, FLAGS, force, verbose)
+    build_host_extension(force, verbose)
+    return lib
 
 
 def _build(objdir: str, lib: str, flags: list[str], force: bool, verbose: bool) -> str:
@@ -63,6 +68,28 @@ def _build(objdir: str, lib: str, flags: list[str], force: bool, verbose: bool) 
     if force or jobs or _stale(lib, objs):
         run([NVCC, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", lib, *objs, "-cudart", "static"])
     return lib
+
+
+def build_host_extension(force: bool = False, verbose: bool = False) -> str:
+    """_host.so: csrc/host_path.cpp against the headers and libraries of the installed torch."""
+    src = os.path.join(CSRC, "host_path.cpp")
+    if not force and not _stale(HOST_EXT, [src, os.path.join(HERE, "..", "include", "shrewq.h")]):
+        return HOST_EXT
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda_inc = os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[a for d in (os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                         sysconfig.get_paths()["include"], cuda_inc) for a in ("-isystem", d)],
+           src, "-o", HOST_EXT, "-L" + os.path.join(root, "lib"), "-Wl,-rpath," + os.path.join(root, "lib"),
+           "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode != 0:
+        sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+    if r.returncode != 0:
+        raise RuntimeError("host extension failed to build: " + " ".join(cmd))
+    return HOST_EXT
 
 
 if __name__ == "__main__":

@@ -149,6 +149,21 @@ _DTYPE_CODE = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16}
 _STORAGE_CODE = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16, torch.float16: _lib.F16, torch.float64: _lib.F64}
 
 
+# members of the enums above as plain names: class attribute lookups are a noticeable part of a short call
+_INT8, _ASYMMETRIC, _PER_CHANNEL = QuantBits.Int8, QuantMode.Asymmetric, QuantGranularity.PerChannel
+
+# CUDA tensors take the compiled host path (csrc/host_path.cpp): the checks, allocations and library calls of the
+# functions below in one C call each.  The Python statements of the same calls remain for tensors that are not on a
+# CUDA device, whose call ends in Device.get's error.
+_host = None
+
+
+def _load_host():
+    global _host
+    _host = _lib.host()
+    return _host
+
+
 # ---- QuantizedTensor (quantize.rs:150-185) -----------------------------------------------------
 @dataclass
 class QuantizedTensor:
@@ -183,6 +198,10 @@ def quantize_tensor(tensor: torch.Tensor, config: QuantConfig) -> QuantizedTenso
     """quantize.rs:194-205 on the GPU.  `tensor` is a float CUDA tensor.  f32 INT8 symmetric runs the
     tuned kernels (shrewq_quantize_f32); the other modes and storage types go through
     shrewq_quantize_f32_ex / shrewq_quantize_any."""
+    if tensor.is_cuda:
+        bits, asym = (8 if config.bits is _INT8 else 4), config.mode is _ASYMMETRIC
+        q, scales, zps, shape = (_host or _load_host()).quantize(tensor, config.granularity is _PER_CHANNEL, bits, asym)
+        return QuantizedTensor(q, scales, shape, tensor.dtype, config, zps)
     dev = Device.get(tensor.device)
     if tensor.dtype not in _STORAGE_CODE:
         raise ShrewError(_lib.ERR_UNSUPPORTED, f"quantize_tensor: dtype {tensor.dtype} is not a float storage type")
@@ -220,6 +239,9 @@ def quantize_tensors(tensors: Sequence[torch.Tensor], config: QuantConfig) -> Li
         return []
     if not config._is_int8_symmetric():
         raise ShrewError(_lib.ERR_UNSUPPORTED, "quantize_tensors: INT8 symmetric only")
+    if tensors[0].is_cuda:
+        return [QuantizedTensor(q, scales, shape, torch.float32, config) for q, scales, shape in
+                (_host or _load_host()).quantize_batch(tensors, config.granularity is _PER_CHANNEL)]
     dev = Device.get(tensors[0].device)
     items = (_lib.QuantItem * len(tensors))()
     out, keep = [], []
@@ -290,6 +312,9 @@ def pack_int4(qtensor: QuantizedTensor) -> torch.Tensor:
 
 def dequantize_tensor(qtensor: QuantizedTensor, device=None) -> torch.Tensor:
     """quantize.rs:210-225 on the GPU: a tensor of the original dtype and shape."""
+    if device is None and qtensor.data.is_cuda:
+        return (_host or _load_host()).dequantize(qtensor.data, qtensor.scales, qtensor.zero_points_t, qtensor.shape,
+                                                  qtensor.config.granularity is _PER_CHANNEL, qtensor.original_dtype)
     dev_t = qtensor.data.device if device is None else torch.device(device)
     dev = Device.get(dev_t)
     out_dtype = qtensor.original_dtype
@@ -361,6 +386,14 @@ class QuantizedLinear:
                                                  weight_q.config.granularity.value, ctypes.byref(h))
         _lib.check(rc, self.device.handle)
         self._h = h
+        self._bind_host()
+
+    def _bind_host(self) -> None:
+        """The compiled counterpart of this handle, for forward and forward_gate_up_silu."""
+        if self.weight_q.data.is_cuda:
+            self._layer = (_host or _load_host()).Layer(self.device.handle.value, self._h.value, self.device.index,
+                                                        self.in_features, self.out_features)
+            self._forward, self._gate_up = self._layer.forward, self._layer.gate_up_silu
 
     @classmethod
     def new(cls, weight_q: QuantizedTensor, bias: Optional[torch.Tensor], device=None) -> "QuantizedLinear":
@@ -386,6 +419,7 @@ class QuantizedLinear:
                                                   ctypes.byref(h))
         _lib.check(rc, self.device.handle)
         self._h = h
+        self._bind_host()
         return self
 
     @classmethod
@@ -431,27 +465,9 @@ class QuantizedLinear:
     def forward(self, x: torch.Tensor, epilogue: int = _lib.EPILOGUE_NONE, out: Optional[torch.Tensor] = None,
                 out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
         """Module::forward (quantize.rs:463-476).  x is [M, in_features] f32 or bf16 on the
-        layer's device; the result has x's dtype.  `out` may be a column slice of a wider
+        layer's device; the result has x's dtype unless out_dtype names another.  `out` may be a column slice of a wider
         row-major buffer (last stride 1): the shard-writes-its-slice case."""
-        if x.dim() != 2 or x.shape[1] != self.in_features:
-            raise ShrewError(_lib.ERR_INVALID_ARG,
-                             f"forward: expected x of shape [M,{self.in_features}], got {list(x.shape)}")
-        if x.dtype not in _DTYPE_CODE:
-            raise ShrewError(_lib.ERR_UNSUPPORTED, f"forward: activation dtype {x.dtype} not supported")
-        if x.device.type != "cuda" or x.device.index != self.device.index:
-            raise ShrewError(_lib.ERR_INVALID_ARG, "forward: x is not on the layer's device")
-        x = x.contiguous()
-        M = x.shape[0]
-        if out is None:
-            out = torch.empty((M, self.out_features), dtype=out_dtype or x.dtype, device=x.device)
-        if out.dim() != 2 or out.shape[0] != M or out.shape[1] != self.out_features or (M > 0 and out.stride(1) != 1):
-            raise ShrewError(_lib.ERR_INVALID_ARG, "forward: bad output buffer")
-        ldy = out.stride(0) if M > 1 else max(out.stride(0), self.out_features)
-        self.device.bind_stream()
-        rc = _lib.lib().shrewq_linear_forward(self._h, _ptr(x), _DTYPE_CODE[x.dtype], M, _ptr(out),
-                                              _DTYPE_CODE[out.dtype], ldy, epilogue)
-        _lib.check(rc, self.device.handle)
-        return out
+        return self._forward(x, epilogue, out, out_dtype)
 
     __call__ = forward
 
@@ -476,16 +492,7 @@ class QuantizedLinear:
 
     def forward_gate_up_silu(self, up: "QuantizedLinear", x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """silu(self.forward(x)) * up.forward(x) in one pass over x (self is the gate)."""
-        x = x.contiguous()
-        M = x.shape[0]
-        if out is None:
-            out = torch.empty((M, self.out_features), dtype=x.dtype, device=x.device)
-        ldh = out.stride(0) if M > 1 else max(out.stride(0), self.out_features)
-        self.device.bind_stream()
-        rc = _lib.lib().shrewq_linear_forward_gate_up_silu(self._h, up._h, _ptr(x), _DTYPE_CODE[x.dtype], M, _ptr(out),
-                                                           _DTYPE_CODE[out.dtype], ldh)
-        _lib.check(rc, self.device.handle)
-        return out
+        return self._gate_up(up._layer, x, out)
 
     def __del__(self):
         h = getattr(self, "_h", None)
