@@ -9,6 +9,7 @@ travel with the source tree; nothing is written outside the package directory.
 from __future__ import annotations
 
 import os
+import re
 import subprocess
 import sys
 import sysconfig
@@ -18,11 +19,21 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libshrewq.so")
 HOST_EXT = os.path.join(HERE, "_host.so")
-SOURCES = ["api.cu", "quantize.cu", "quantize_batch.cu", "quantize_modes.cu", "gemv.cu", "gemv_mma.cu", "gemm_simt.cu", "gemm_tcgen05.cu", "gemm_tcgen05_2cta.cu", "exchange.cu"]
-HEADERS = sorted(os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith(".cuh")) + [os.path.join(HERE, "..", "include", "shrewq.h")]
+SOURCES = ["api.cu", "quantize.cu", "quantize_batch.cu", "quantize_modes.cu", "gemv.cu", "gemv_mma.cu", "gemm_simt.cu", "gemm_tcgen05.cu", "gemm_tcgen05_g1.cu", "gemm_tcgen05_g2.cu", "gemm_tcgen05_g3.cu", "gemm_tcgen05_2cta.cu", "exchange.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
          "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
+
+
+def _includes(path: str, seen: set | None = None) -> list[str]:
+    """The file and every header it includes by a quoted name, transitively: what its object depends on."""
+    seen = set() if seen is None else seen
+    if path not in seen and os.path.exists(path):
+        seen.add(path)
+        with open(path) as f:
+            for name in re.findall(r'^\s*#\s*include\s+"([^"]+)"', f.read(), flags=re.M):
+                _includes(os.path.normpath(os.path.join(os.path.dirname(path), name)), seen)
+    return sorted(seen)
 
 
 def _stale(target: str, deps: list[str]) -> bool:
@@ -49,7 +60,7 @@ def _build(objdir: str, lib: str, flags: list[str], force: bool, verbose: bool) 
     for src in SOURCES:
         s = os.path.join(CSRC, src)
         o = os.path.join(objdir, src.replace(".cu", ".o"))
-        if force or _stale(o, [s] + HEADERS):
+        if force or _stale(o, _includes(s)):
             cmd = [NVCC, *flags, "-c", s, "-o", o]
             if verbose:
                 cmd.insert(1, "-Xptxas=-v")
@@ -73,7 +84,7 @@ def _build(objdir: str, lib: str, flags: list[str], force: bool, verbose: bool) 
 def build_host_extension(force: bool = False, verbose: bool = False) -> str:
     """_host.so: csrc/host_path.cpp against the headers and libraries of the installed torch."""
     src = os.path.join(CSRC, "host_path.cpp")
-    if not force and not _stale(HOST_EXT, [src, os.path.join(HERE, "..", "include", "shrewq.h")]):
+    if not force and not _stale(HOST_EXT, _includes(src)):
         return HOST_EXT
     import torch
     root = os.path.dirname(torch.__file__)

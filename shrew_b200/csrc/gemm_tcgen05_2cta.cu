@@ -80,10 +80,6 @@ int launch_pair(shrewq_ctx *ctx, const ForwardArgs &a, const CUtensorMap &tw, co
             const int splits_t = (rounds + rps_t - 1) / rps_t;
             const size_t part_bytes = (size_t)2 * rem * splits_t * kTokPair * kLanes * sizeof(float);
             if ((rc = ensure_scratch(ctx, 8192 + part_bytes)) != SHREWQ_OK) return rc;
-            if (!ctx->counters_zeroed) {
-                SHREWQ_CUDA_TRY(ctx, cudaMemsetAsync(static_cast<char *>(ctx->scratch) + 4096, 0, 4096, ctx->stream));
-                ctx->counters_zeroed = true;
-            }
             SplitK2 head{nullptr, nullptr, rounds, 0, (int)pairs};
             SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(kern, dim3(2u * (unsigned)(tiles - rem), 1, 1), dim3(kThreads), (size_t)kSmemBytes,
                                                   ctx->stream, a.pdl, tw, tw2, tx, ops, static_cast<YT *>(a.y), a.extra, (int)a.M,
@@ -104,10 +100,6 @@ int launch_pair(shrewq_ctx *ctx, const ForwardArgs &a, const CUtensorMap &tw, co
         // context scratch as in the single-CTA launcher: tile counters at 4096, partial sums from 8192
         const size_t part_bytes = (size_t)ctas * splits * kTokPair * kLanes * sizeof(float);
         if ((rc = ensure_scratch(ctx, 8192 + part_bytes)) != SHREWQ_OK) return rc;
-        if (!ctx->counters_zeroed) {
-            SHREWQ_CUDA_TRY(ctx, cudaMemsetAsync(static_cast<char *>(ctx->scratch) + 4096, 0, 4096, ctx->stream));
-            ctx->counters_zeroed = true;
-        }
         sk.counters = reinterpret_cast<unsigned int *>(static_cast<char *>(ctx->scratch) + 4096);
         sk.partials = reinterpret_cast<float *>(static_cast<char *>(ctx->scratch) + 8192);
     }
