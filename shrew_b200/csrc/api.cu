@@ -49,8 +49,11 @@ int ensure_scratch(shrewq_ctx *ctx, size_t bytes) {
     const void *before = ctx->scratch;
     // never smaller than the fixed head (quantizer words + split-K tile counters)
     int rc = grow(ctx, &ctx->scratch, &ctx->scratch_bytes, bytes < 8192 ? 8192 : bytes, false);
-    if (ctx->scratch != before) ctx->counters_zeroed = false;  // new memory: counters are garbage
-    return rc;
+    if (rc != SHREWQ_OK || ctx->scratch == before) return rc;
+    // the head's counters start at zero; the kernels leave them at zero
+    SHREWQ_CUDA_TRY(ctx, cudaMemsetAsync(ctx->scratch, 0, 8192, ctx->stream));
+    SHREWQ_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    return SHREWQ_OK;
 }
 
 int ensure_xsplit(shrewq_ctx *ctx, size_t bytes) { return grow(ctx, &ctx->xsplit, &ctx->xsplit_bytes, bytes, false); }

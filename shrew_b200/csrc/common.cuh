@@ -40,11 +40,9 @@ struct shrewq_ctx {
     char err[shrewq::kErrLen] = {0};
     std::atomic<uint64_t> launches{0};
     shrewq::Tuning tuning;
-    // scratch: per-tensor amax word, split-K partial sums and tile counters
+    // scratch: quantizer words, split-K tile counters (both zeroed with the allocation, left at zero by the kernels), partial sums
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
-    // split-K tile counters live in scratch; they are zeroed once and reset by the kernels
-    bool counters_zeroed = false;
     // the gated block's host-buffer entry point: two staging slots and two copy streams, so that the copies of
     // one call overlap the kernels of its neighbours (created on first use)
     cudaStream_t copy_in = nullptr, copy_out = nullptr;

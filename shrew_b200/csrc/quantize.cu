@@ -1,68 +1,125 @@
 // Launchers of the INT8 symmetric quantize / dequantize kernels (device code and its description:
 // quantize_kernels.cuh).
+#include <cuda_fp16.h>
+
 #include "common.cuh"
 #include "quantize_kernels.cuh"
+#include "quantize_launch.cuh"
 
 namespace shrewq {
 
 namespace {
 
-template <int GROUP, int NV>
-void launch_rows_reg(shrewq_ctx *ctx, const float *w, size_t rows, size_t cols, int8_t *q, double *scales) {
-    constexpr int THREADS = GROUP >= 256 ? GROUP : 256;
-    constexpr int ROWS_PER_CTA = THREADS / GROUP;
-    const unsigned grid = (unsigned)((rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA);
-    quantize_rows_reg_kernel<GROUP, NV><<<grid, THREADS, 0, ctx->stream>>>(w, rows, cols, q, scales);
+template <int GROUP, int NV, typename T, bool ASYM>
+void rows_reg(shrewq_ctx *ctx, const T *w, size_t rows, size_t cols, int8_t *q, double *scales, double *zps, int bits) {
+    constexpr int THREADS = GROUP == 32 ? 256 : GROUP;
+    constexpr size_t kRows = GROUP == 32 ? 8 * (8 / NV) : 1;  // rows per CTA
+    const size_t grid = (rows + kRows - 1) / kRows;
+    launch_maybe_pdl(quantize_rows_reg_kernel<GROUP, NV, T, ASYM>, dim3((unsigned)grid), dim3(THREADS), 0, ctx->stream, true, w, rows, cols, q, scales, zps,
+                     bits);
+}
+
+template <int GROUP, int NE, typename T, bool ASYM>
+void rows_elem(shrewq_ctx *ctx, const T *w, size_t rows, size_t cols, int8_t *q, double *scales, double *zps, int bits) {
+    const unsigned grid = (unsigned)(GROUP == 32 ? (rows + 7) / 8 : rows);
+    launch_maybe_pdl(quantize_rows_elem_kernel<GROUP, NE, T, ASYM>, dim3(grid), dim3(GROUP == 32 ? 256 : GROUP), 0, ctx->stream, true, w, rows, cols, q,
+                     scales, zps, bits);
+}
+
+// Per-channel rows through registers.  false: the row is too long for it.
+template <typename T, bool ASYM>
+bool rows_in_registers(shrewq_ctx *ctx, const T *w, size_t rows, size_t cols, int bits, int8_t *q, double *scales, double *zps) {
+    constexpr int EPV = Vec16<T>::kElems;
+    const bool vec = cols % EPV == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && (reinterpret_cast<uintptr_t>(q) & (EPV - 1)) == 0;
+    const size_t nvec = cols / EPV;
+    // Tile widths by the vectors of a row: a warp up to 256 of them, then whole CTAs.  f32 rows of more than 1024 vectors keep
+    // eight per thread (98 % of the copy rate); the 16-bit types, with twice the elements in a vector, keep four.
+    constexpr bool k16 = sizeof(T) == 2;
+    if (vec && nvec <= 32) rows_reg<32, 1, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else if (vec && nvec <= 64) rows_reg<32, 2, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else if (vec && nvec <= 128) rows_reg<32, 4, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else if (vec && nvec <= 256) rows_reg<32, 8, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else if (vec && nvec <= 512) rows_reg<k16 ? 128 : 256, k16 ? 4 : 2, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else if (vec && nvec <= 1024) rows_reg<256, 4, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else if (vec && nvec <= 2048) rows_reg<k16 ? 512 : 256, k16 ? 4 : 8, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else if (vec && nvec <= 4096) rows_reg<k16 ? 1024 : 512, k16 ? 4 : 8, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else if (vec && nvec <= 8192) rows_reg<1024, 8, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    // element tiles: the narrowest that holds the row (its unused slots cost as much as used ones)
+    else if (cols <= 256) rows_elem<32, 8, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else if (cols <= 512) rows_elem<32, 16, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else if (cols <= 1024) rows_elem<128, 8, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else if (cols <= 2048) rows_elem<256, 8, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else if (cols <= 4096) rows_elem<256, 16, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else if (cols <= 8192) rows_elem<512, 16, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
+    else return false;
+    ctx->launches += 1;
+    return true;
+}
+
+// Per-tensor in two launches (extrema and parameters, codes), the second one allowed to start under the first one's tail.
+template <typename T, bool ASYM>
+int tensor_two_pass(shrewq_ctx *ctx, const T *w, size_t n, int bits, int8_t *q, double *scales, double *zps) {
+    // scratch: the arrival counter in the head that is zeroed with the allocation, the rest where split-K keeps partial sums
+    int rc = ensure_scratch(ctx, 8192 + sizeof(TensorGroup));
+    if (rc != SHREWQ_OK) return rc;
+    unsigned int *arrived = reinterpret_cast<unsigned int *>(static_cast<char *>(ctx->scratch) + 4032);
+    TensorGroup *g = reinterpret_cast<TensorGroup *>(static_cast<char *>(ctx->scratch) + 8192);
+    const size_t vecs = n / Vec16<T>::kElems;
+    const size_t cap = (size_t)ctx->sm_count * 8 < (size_t)kMaxPartials ? (size_t)ctx->sm_count * 8 : (size_t)kMaxPartials;
+    const size_t want = (vecs + 1023) / 1024;
+    SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(extrema_partials_kernel<T, ASYM>, dim3((unsigned)(want < 1 ? 1 : (want > cap ? cap : want))), dim3(256), 0,
+                                          ctx->stream, true, w, n, bits, g, arrived, scales, zps));
+    ctx->launches += 1;
+    if (n > 0) {
+        constexpr int U = sizeof(T) == 2 ? 2 : 4;
+        SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(quantize_tensor_kernel<T, ASYM, U>, dim3((unsigned)(want < 1 ? 1 : (vecs + 256 * U - 1) / (256 * U))),
+                                              dim3(256), 0, ctx->stream, true, w, n, static_cast<const TensorGroup *>(g), q));
+        ctx->launches += 1;
+    }
+    return SHREWQ_OK;
+}
+
+template <typename T, bool ASYM>
+int quantize_t(shrewq_ctx *ctx, const T *w, size_t rows, size_t cols, int granularity, int bits, int8_t *q, double *scales,
+               double *zps, bool *taken) {
+    *taken = true;
+    if (granularity == SHREWQ_PER_CHANNEL) {
+        if (rows == 0) return SHREWQ_OK;
+        if (rows > 0x7FFFFFFFull) return set_err(ctx, SHREWQ_ERR_UNSUPPORTED, "quantize: more than 2^31-1 channels");
+        *taken = rows_in_registers<T, ASYM>(ctx, w, rows, cols, bits, q, scales, zps);
+    } else {
+        int rc = tensor_two_pass<T, ASYM>(ctx, w, rows * cols, bits, q, scales, zps);
+        if (rc != SHREWQ_OK) return rc;
+    }
+    SHREWQ_CUDA_TRY(ctx, cudaGetLastError());
+    return SHREWQ_OK;
 }
 
 }  // namespace
 
+// f32, bf16 or f16 tensors in any mode.  *taken false: per-channel rows too long for the register kernels.
+int launch_quantize_tuned(shrewq_ctx *ctx, const void *w, int w_dtype, size_t rows, size_t cols, int granularity, int bits,
+                          int mode, int8_t *q, double *scales, double *zps, bool *taken) {
+    const bool asym = mode == SHREWQ_ASYMMETRIC;
+#define SHREWQ_QUANT(T)                                                                                                          \
+    return asym ? quantize_t<T, true>(ctx, static_cast<const T *>(w), rows, cols, granularity, bits, q, scales, zps, taken)     \
+                : quantize_t<T, false>(ctx, static_cast<const T *>(w), rows, cols, granularity, bits, q, scales, zps, taken)
+    if (w_dtype == SHREWQ_F32) SHREWQ_QUANT(float);
+    if (w_dtype == SHREWQ_BF16) SHREWQ_QUANT(__nv_bfloat16);
+    if (w_dtype == SHREWQ_F16) SHREWQ_QUANT(__half);
+#undef SHREWQ_QUANT
+    *taken = false;
+    return SHREWQ_OK;
+}
+
 int launch_quantize(shrewq_ctx *ctx, const float *w, size_t rows, size_t cols, int granularity,
                     int8_t *q, double *scales) {
-    const size_t n = rows * cols;
-    if (granularity == SHREWQ_PER_CHANNEL) {
-        if (rows == 0) return SHREWQ_OK;
-        if (rows > 0x7FFFFFFFull) return set_err(ctx, SHREWQ_ERR_UNSUPPORTED, "quantize: more than 2^31-1 channels");
-        const bool vec = (cols % 4 == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0) &&
-                         ((reinterpret_cast<uintptr_t>(q) & 3) == 0) && cols >= 32;
-        if (vec && cols <= 128) launch_rows_reg<32, 1>(ctx, w, rows, cols, q, scales);
-        else if (vec && cols <= 256) launch_rows_reg<32, 2>(ctx, w, rows, cols, q, scales);
-        else if (vec && cols <= 512) launch_rows_reg<32, 4>(ctx, w, rows, cols, q, scales);
-        else if (vec && cols <= 1024) launch_rows_reg<32, 8>(ctx, w, rows, cols, q, scales);
-        else if (vec && cols <= 2048) launch_rows_reg<256, 2>(ctx, w, rows, cols, q, scales);
-        else if (vec && cols <= 4096) launch_rows_reg<256, 4>(ctx, w, rows, cols, q, scales);
-        else if (vec && cols <= 8192) launch_rows_reg<256, 8>(ctx, w, rows, cols, q, scales);
-        // 512 threads x 8 float4 rather than 256 x 16: 48 registers per thread instead of 80 keeps
-        // more rows resident per SM (the 256 x 16 tile measured 4.4 TB/s against 5.1-5.5 TB/s for
-        // the 8-float4 tiles)
-        else if (vec && cols <= 16384) launch_rows_reg<512, 8>(ctx, w, rows, cols, q, scales);
-        else if (vec && cols <= 32768) launch_rows_reg<1024, 8>(ctx, w, rows, cols, q, scales);
-        else {
-            const unsigned grid = (unsigned)(rows < (size_t)ctx->sm_count * 32 ? rows : (size_t)ctx->sm_count * 32);
-            quantize_rows_generic_kernel<<<grid, 256, 0, ctx->stream>>>(w, rows, cols, q, scales);
-        }
-        ctx->launches += 1;
-    } else {
-        // scratch layout: [0] amax bits, [64..] TensorParams
-        int rc = ensure_scratch(ctx, 256);
-        if (rc != SHREWQ_OK) return rc;
-        unsigned int *amax_bits = reinterpret_cast<unsigned int *>(ctx->scratch);
-        TensorParams *tp = reinterpret_cast<TensorParams *>(reinterpret_cast<char *>(ctx->scratch) + 64);
-        SHREWQ_CUDA_TRY(ctx, cudaMemsetAsync(amax_bits, 0, 4, ctx->stream));
-        size_t want = (n / 4 + 255) / 256;
-        const size_t cap = (size_t)ctx->sm_count * 16;
-        unsigned grid = (unsigned)(want < 1 ? 1 : (want > cap ? cap : want));
-        if (n > 0) {
-            absmax_flat_kernel<<<grid, 256, 0, ctx->stream>>>(w, n, amax_bits);
-            ctx->launches += 1;
-        }
-        finalize_tensor_scale_kernel<<<1, 1, 0, ctx->stream>>>(amax_bits, n, scales, tp);
-        ctx->launches += 1;
-        if (n > 0) {
-            quantize_flat_kernel<<<grid, 256, 0, ctx->stream>>>(w, n, tp, q);
-            ctx->launches += 1;
-        }
-    }
+    bool taken = false;
+    int rc = launch_quantize_tuned(ctx, w, SHREWQ_F32, rows, cols, granularity, 8, SHREWQ_SYMMETRIC, q, scales, nullptr, &taken);
+    if (rc != SHREWQ_OK || taken) return rc;
+    const unsigned grid = (unsigned)(rows < (size_t)ctx->sm_count * 32 ? rows : (size_t)ctx->sm_count * 32);
+    quantize_rows_generic_kernel<<<grid, 256, 0, ctx->stream>>>(w, rows, cols, q, scales);
+    ctx->launches += 1;
     SHREWQ_CUDA_TRY(ctx, cudaGetLastError());
     return SHREWQ_OK;
 }
@@ -110,17 +167,17 @@ int launch_dequantize(shrewq_ctx *ctx, const int8_t *q, const double *scales, si
     const size_t n = rows * cols;
     if (n == 0) return SHREWQ_OK;
     const int per_channel = granularity == SHREWQ_PER_CHANNEL;
-    const int vec_ok = (cols % 4 == 0) && ((reinterpret_cast<uintptr_t>(q) & 3) == 0) &&
-                       ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
-    size_t want = ((vec_ok ? n / 4 : n) + 255) / 256;
-    const size_t cap = (size_t)ctx->sm_count * 32;
+    const int vec_ok = ((reinterpret_cast<uintptr_t>(q) & 3) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
+    const size_t words = 256 * (out_dtype == SHREWQ_F32 ? DequantWords<float>::kPerThread : DequantWords<uint16_t>::kPerThread);
+    const size_t want = vec_ok ? (n / 4 + words - 1) / words : (n + 255) / 256;
+    const size_t cap = vec_ok ? 0x7FFFFFFF : (size_t)ctx->sm_count * 32;
     unsigned grid = (unsigned)(want < 1 ? 1 : (want > cap ? cap : want));
     if (out_dtype == SHREWQ_F32)
-        dequantize_kernel<float><<<grid, 256, 0, ctx->stream>>>(q, scales, rows, cols, per_channel,
-                                                                 static_cast<float *>(out), vec_ok);
+        SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(dequantize_kernel<float>, dim3(grid), dim3(256), 0, ctx->stream, true, q, scales, rows, cols, per_channel,
+                                              static_cast<float *>(out), vec_ok));
     else
-        dequantize_kernel<uint16_t><<<grid, 256, 0, ctx->stream>>>(q, scales, rows, cols, per_channel,
-                                                                    static_cast<uint16_t *>(out), vec_ok);
+        SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(dequantize_kernel<uint16_t>, dim3(grid), dim3(256), 0, ctx->stream, true, q, scales, rows, cols, per_channel,
+                                              static_cast<uint16_t *>(out), vec_ok));
     ctx->launches += 1;
     SHREWQ_CUDA_TRY(ctx, cudaGetLastError());
     return SHREWQ_OK;

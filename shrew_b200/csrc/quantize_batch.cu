@@ -27,17 +27,19 @@ int launch_quantize_batch(shrewq_ctx *ctx, const shrewq_quant_item *items, size_
                                                             "quantize the large tensors one by one");
         }
         t.total_units = (unsigned int)units;
-        const unsigned long long want = (units + kBatchWarps - 1) / kBatchWarps;
+        // a warp takes four rows (per-channel) or one segment (per-tensor) at a time
+        const unsigned long long per_cta = kBatchWarps * (per_channel ? 4ull : 1ull);
+        const unsigned long long want = (units + per_cta - 1) / per_cta;
         const unsigned long long cap = (unsigned long long)ctx->sm_count * 16;
         const unsigned grid = (unsigned)(want < 1 ? 1 : (want > cap ? cap : want));
         if (per_channel) {
             if (units > 0) {
-                quantize_batch_rows_kernel<<<grid, kBatchWarps * 32, 0, ctx->stream>>>(t);
+                SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(quantize_batch_rows_kernel, dim3(grid), dim3(kBatchWarps * 32), 0, ctx->stream, true, t));
                 ctx->launches += 1;
             }
         } else {
             // scratch: one amax word per tensor at [0, 256), one TensorParams per tensor from 256
-            static_assert(kBatchMax * sizeof(unsigned int) <= 256 && 256 + kBatchMax * sizeof(TensorParams) <= 4096,
+            static_assert(kBatchMax * sizeof(unsigned int) <= 256 && 256 + kBatchMax * sizeof(TensorParams) <= 4032,
                           "the quantizer's part of the context scratch is its first 4096 bytes");
             int rc = ensure_scratch(ctx, 4096);
             if (rc != SHREWQ_OK) return rc;

@@ -1,33 +1,23 @@
-// INT8 symmetric quantize / dequantize kernels (sm_100a).
+// Quantize / dequantize kernels (sm_100a): per-channel rows of f32, bf16 or f16 in every mode, per-tensor, and back.
 //
-// Reference semantics (crates/shrew/src/quantize.rs):
-//   scale     = amax < 1e-30 ? 1.0 : amax / 127.0                (f64, :349-351)
-//   inv_scale = |scale| < 1e-30 ? 0.0 : 1.0 / scale              (f64, :236-240, :295-299)
-//   code      = clamp(round_half_away(v * inv_scale + 0.0), -127, 127) as i8   (:244-250)
-// all in f64 on a widened copy of the f32 tensor.  The kernels below produce the same
-// bits.  amax of f32 values is exact in f32.  The element map runs in f32 and is trusted
-// only when the product lies far from a rounding boundary; the few elements near a
-// boundary (and every element of a row whose inv_scale is not an ordinary f32 number) are
-// recomputed with the reference's exact f64 operations.  Why that is safe: for |t| <= 127
-// the f32 product differs from the f64 one by at most 127 * 2^-23 ~ 1.5e-5, and the
-// recompute window is 1e-4 on either side of x.5.
+// The arithmetic, and why the f32 shortcut gives the reference's f64 codes bit for bit: quantize_common.cuh.
 //
-// Memory plan (HBM-bound, 5 B/element algorithmic): a row is read ONCE into registers,
-// reduced (warp shuffles, then shared memory across warps), and quantized from registers;
-// codes are written as packed 32-bit words.  Rows too long for registers take a two-pass
-// kernel whose second read normally hits L2.
+// Memory plan (HBM-bound; f32 5 B/element, bf16 and f16 3 B/element): a row is read ONCE into registers as 16-byte
+// vectors, reduced (warp shuffles, then shared memory across warps), and quantized from registers; codes are
+// written as packed words.  Rows that are not whole aligned vectors are held in registers element by element; rows
+// too long for registers take a two-pass kernel whose second read normally hits L2.  Per-tensor: one pass for the
+// extrema of every block, a second one for the codes.
+//
+// The kernels are launched with programmatic stream serialization and wait for the previous kernel before they touch
+// memory: the next launch's start-up lies under the tail of the one before.
 //
 // This header holds the device code only (no launch syntax, no runtime calls), so that it also
 // compiles as plain C++ against a small CUDA stand-in: the CPU tests run these kernels thread by
 // thread and compare them with the golden vectors (tests/cpu_emu/).
 #pragma once
 
-#include "../../include/shrewq.h"
-#ifndef SHREWQ_CPU_EMU
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
-#include <stdint.h>
-#endif
+#include "ptx_small.cuh"
+#include "quantize_common.cuh"
 
 namespace shrewq {
 namespace {
@@ -59,15 +49,12 @@ __device__ __forceinline__ int quant_exact(float v, double inv64) {
     return (int)r;
 }
 
+// for scales that do not come from the elements themselves (a supplied amax): the f32 candidate is clamped
 __device__ __forceinline__ int quant_one(float v, const RowParams &p) {
     if (!p.exact_only) {
-        float t = v * p.inv32;
-        float a = fabsf(t);
-        float frac = a - truncf(a);  // exact
-        if (fabsf(frac - 0.5f) > 1e-4f && a < 1000.0f) {  // false for NaN
-            int m = min((int)(a + 0.5f), 127);
-            return t < 0.0f ? -m : m;
-        }
+        const float t = v * p.inv32, a = t + kRoundMagic;
+        if (fabsf(t - (a - kRoundMagic)) <= kSafeSym && fabsf(t) < 1000.0f)  // false for NaN
+            return max(-127, min(127, (int)(__float_as_uint(a) - __float_as_uint(kRoundMagic))));
     }
     return quant_exact(v, p.inv64);
 }
@@ -89,68 +76,153 @@ __device__ __forceinline__ float warp_max(float v) {
 }
 
 // ---- per-channel, row held in registers ---------------------------------------------
-// GROUP threads own one row; each keeps NV float4.  cols % 4 == 0, pointers 16 B / 4 B
-// aligned (checked by the launcher).
-template <int GROUP, int NV>
-__global__ void __launch_bounds__(GROUP >= 256 ? GROUP : 256)
-quantize_rows_reg_kernel(const float *__restrict__ w, size_t rows, size_t cols,
-                         int8_t *__restrict__ q, double *__restrict__ scales) {
-    constexpr int THREADS = GROUP >= 256 ? GROUP : 256;
-    constexpr int ROWS_PER_CTA = THREADS / GROUP;
-    constexpr int WARPS_PER_GROUP = GROUP / 32;
-    const int g = threadIdx.x / GROUP;
-    const int t = threadIdx.x % GROUP;
-    const size_t row = (size_t)blockIdx.x * ROWS_PER_CTA + g;
-    const bool active = row < rows;
-    const int nvec = (int)(cols >> 2);
-    const float4 *src = reinterpret_cast<const float4 *>(w + (active ? row : 0) * cols);
-
-    float4 v[NV];
-    float amax = 0.0f;
+// The extrema of a row from those of its threads.  GROUP threads own a row; with several warps per row they meet in
+// shared memory (one barrier; every thread reads the partial results itself, so no second one is needed).
+template <int GROUP, bool ASYM>
+__device__ __forceinline__ void extrema_group(Extrema &e, int t) {
+    constexpr int W = GROUP / 32;
+    __shared__ Extrema s_part[W];
+    extrema_warp<ASYM>(e);
+    if ((t & 31) == 0) s_part[t >> 5] = e;
+    __syncthreads();
+    if constexpr (W <= 8) {
+        e = s_part[0];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-        const int c = t + i * GROUP;
-        v[i] = (active && c < nvec) ? __ldcs(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-#pragma unroll
-    for (int i = 0; i < NV; ++i) amax = fmaxf(amax, abs4max(v[i]));
-    amax = warp_max(amax);
-
-    RowParams p;
-    if constexpr (WARPS_PER_GROUP == 1) {
-        double scale;
-        make_params(amax, &scale, &p);  // every lane: 2 f64 divisions, rows here are short
-        if (active && t == 0) scales[row] = scale;
+        for (int i = 1; i < W; ++i) extrema_merge<ASYM>(e, s_part[i]);
     } else {
-        __shared__ float s_part[THREADS / 32];
-        __shared__ RowParams s_p[ROWS_PER_CTA];
-        const int wig = t >> 5;  // warp in group
-        if ((t & 31) == 0) s_part[g * WARPS_PER_GROUP + wig] = amax;
-        __syncthreads();
-        if (t < 32) {
-            float m = 0.0f;
-            for (int i = t; i < WARPS_PER_GROUP; i += 32) m = fmaxf(m, s_part[g * WARPS_PER_GROUP + i]);
-            m = warp_max(m);
-            if (t == 0) {
-                double scale;
-                RowParams pp;
-                make_params(m, &scale, &pp);
-                s_p[g] = pp;
-                if (active) scales[row] = scale;
+        e = s_part[(t & 31) < W ? (t & 31) : 0];
+        extrema_warp<ASYM>(e);
+    }
+}
+
+// GROUP = 32: a warp takes 8 / NV consecutive rows at a time.  Otherwise the GROUP threads of a CTA own one row, NV
+// 16-byte vectors each.  cols is a multiple of the vector's elements, w is 16-byte and q 4-byte (f32) or 8-byte aligned
+// (checked by the launcher).  Thread 0 forms the f64 parameters while the others already write codes; the undecided
+// elements wait for them at the end (symmetric; an asymmetric row's zero point is needed for every code).
+// 8192 x 8192 f32: 52 us (6.4 TB/s); 66.9 us with two barriers a row, two f64 divisions on the way to the codes and ~20
+// instructions an element.  (CTAs that walk over rows with the next row's loads in flight were slower: 33 against 29 us
+// for 8192 x 4096, the registers cost more resident rows than the look-ahead gave.)
+template <int GROUP, int NV, typename T = float, bool ASYM = false>
+__global__ void __launch_bounds__(GROUP == 32 ? 256 : GROUP)
+quantize_rows_reg_kernel(const T *__restrict__ w, size_t rows, size_t cols, int8_t *__restrict__ q, double *__restrict__ scales,
+                         double *__restrict__ zps = nullptr, int bits = 8) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int EPV = Vec16<T>::kElems;
+    if constexpr (GROUP == 32) {
+        constexpr int R = NV >= 8 ? 1 : 8 / NV;
+        const size_t row = ((size_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * R;
+        if (row >= rows) return;
+        const int count = rows - row < (size_t)R ? (int)(rows - row) : R;
+        quantize_rows_by_warp<R, NV, T, ASYM>(w + row * cols, cols, count, bits, q + row * cols, scales + row, zps ? zps + row : zps,
+                                              threadIdx.x & 31);
+    } else {
+        const int t = threadIdx.x;
+        const size_t row = blockIdx.x;
+        const int nvec = (int)(cols / EPV);
+        const T *src = w + row * cols;
+        int8_t *dst = q + row * cols;
+        __shared__ GroupParams s_p;
+        uint4 v[NV];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int c = t + i * GROUP;
+            v[i] = c < nvec ? __ldcs(reinterpret_cast<const uint4 *>(src) + c) : make_uint4(0, 0, 0, 0);
+        }
+        Extrema e = extrema_none<ASYM>();
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+            if (!ASYM || t + i * GROUP < nvec) extrema_add16<T, ASYM>(e, v[i]);  // (amax does not mind the zeros)
+        extrema_group<GROUP, ASYM>(e, t);
+        if (t == 0) {
+            s_p = group_of<ASYM>(e, cols, bits);
+            scales[row] = s_p.scale;
+            if (zps) zps[row] = s_p.zp;
+        }
+        if constexpr (ASYM) __syncthreads();
+        const FastGroup f = fast_of<ASYM>(e, bits, ASYM ? s_p.zp : 0.0);
+        constexpr int H = (NV * EPV + 31) / 32;
+        uint32_t redo[H] = {0};
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int c = t + i * GROUP;
+            if (c >= nvec) break;
+            float x[EPV];
+            uint32_t word[EPV / 4];
+            unpack16(v[i], static_cast<const T *>(nullptr), x);
+            redo[i * EPV / 32] |= quant_words<ASYM, EPV>(x, f, word) << (i * EPV % 32);
+            store_codes<EPV>(dst, c, word);
+            if (f.exact) redo[i * EPV / 32] |= ((1u << EPV) - 1u) << (i * EPV % 32);
+        }
+        if constexpr (!ASYM) __syncthreads();
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+#pragma unroll 1
+            for (uint32_t left = redo[h]; left != 0; left &= left - 1) {
+                const int k = h * 32 + lowest_bit(left);
+                const size_t at = (size_t)(t + k / EPV * GROUP) * EPV + k % EPV;
+                dst[at] = (int8_t)quant_ex(widen(src[at]), s_p);
             }
         }
-        __syncthreads();
-        p = s_p[g];
     }
+}
 
-    if (!active) return;
-    uint32_t *dst = reinterpret_cast<uint32_t *>(q + row * cols);
+// Rows that are not whole aligned vectors: the same with NE elements per thread, consecutive threads on consecutive
+// elements (a warp's loads are 32 elements, its stores 32 bytes).  GROUP = 32: a row per warp, else a row per CTA.
+template <int GROUP, int NE, typename T, bool ASYM>
+__global__ void __launch_bounds__(GROUP == 32 ? 256 : GROUP)
+quantize_rows_elem_kernel(const T *__restrict__ w, size_t rows, size_t cols, int8_t *__restrict__ q, double *__restrict__ scales,
+                          double *__restrict__ zps, int bits) {
+    pdl_launch_dependents();
+    pdl_wait();
+    static_assert(NE <= 32, "one mask bit per element");
+    constexpr int kRows = GROUP == 32 ? 8 : 1;  // rows per CTA
+    const int t = threadIdx.x % GROUP;
+    const size_t row = (size_t)blockIdx.x * kRows + threadIdx.x / GROUP;
+    if (GROUP == 32 && row >= rows) return;
+    const int n = (int)cols;
+    const T *src = w + row * cols;
+    int8_t *dst = q + row * cols;
+    __shared__ GroupParams s_p[kRows];
+    float v[NE];
+    Extrema e = extrema_none<ASYM>();
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
+    for (int i = 0; i < NE; ++i) {
         const int c = t + i * GROUP;
-        if (c < nvec)
-            __stcs(dst + c, pack4(quant_one(v[i].x, p), quant_one(v[i].y, p), quant_one(v[i].z, p),
-                                  quant_one(v[i].w, p)));
+        v[i] = c < n ? storage_to_f32(__ldcs(src + c)) : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < NE; ++i)
+        if (!ASYM || t + i * GROUP < n) extrema_add<ASYM>(e, v[i]);
+    GroupParams &p = s_p[threadIdx.x / GROUP];
+    if constexpr (GROUP == 32) extrema_warp<ASYM>(e);
+    else extrema_group<GROUP, ASYM>(e, t);
+    if (t == 0) {
+        p = group_of<ASYM>(e, cols, bits);
+        scales[row] = p.scale;
+        if (zps) zps[row] = p.zp;
+    }
+    if constexpr (ASYM) {
+        if constexpr (GROUP == 32) __syncwarp();
+        else __syncthreads();
+    }
+    const FastGroup f = fast_of<ASYM>(e, bits, ASYM ? p.zp : 0.0);
+    uint32_t redo = f.exact ? ~0u : 0u;
+#pragma unroll
+    for (int i = 0; i < NE; ++i) {
+        const int c = t + i * GROUP;
+        uint32_t m;
+        if (undecided<ASYM>(quant_candidate<ASYM>(v[i], f, m))) redo |= 1u << i;
+        if (c < n) dst[c] = (int8_t)m;
+    }
+    if constexpr (!ASYM) {
+        if constexpr (GROUP == 32) __syncwarp();
+        else __syncthreads();
+    }
+#pragma unroll 1
+    for (uint32_t left = redo; left != 0; left &= left - 1) {
+        const int i = lowest_bit(left), c = t + i * GROUP;
+        if (i < NE && c < n) dst[c] = (int8_t)quant_ex(widen(src[c]), p);
     }
 }
 
@@ -208,6 +280,108 @@ absmax_flat_kernel(const float *__restrict__ w, size_t n, unsigned int *amax_bit
     }
 }
 
+// Per-tensor in two launches.  Every block leaves the extrema of its contiguous part; the block that finishes last
+// reduces them and forms the tensor's parameters, so no kernel of one thread sits between the passes and nothing has
+// to be cleared (the counter wraps to zero by itself).  The second pass takes the tensor from its end, where the
+// first one stopped: that much of it may still be in L2.
+constexpr int kMaxPartials = 2048;
+
+struct TensorGroup {
+    GroupParams p;
+    FastGroup f;
+    alignas(16) Extrema partials[kMaxPartials];  // read as float2
+};
+static_assert(sizeof(Extrema) == 8, "an Extrema is two floats");
+
+#ifndef SHREWQ_CPU_EMU  // (the CPU model has no wrapping atomic)
+template <typename T, bool ASYM>
+__global__ void __launch_bounds__(256)
+extrema_partials_kernel(const T *__restrict__ w, size_t n, int bits, TensorGroup *g, unsigned int *arrived, double *__restrict__ scales,
+                        double *__restrict__ zps) {
+    // in this order: the second launch reads w before its own wait, so none of it may start before w is complete
+    pdl_wait();
+    pdl_launch_dependents();
+    constexpr int EPV = Vec16<T>::kElems;
+    __shared__ unsigned int s_last;
+    Extrema e = extrema_none<ASYM>();
+    const size_t nvec = (reinterpret_cast<uintptr_t>(w) & 15) == 0 ? n / EPV : 0;
+    const uint4 *w4 = reinterpret_cast<const uint4 *>(w);
+    const size_t stride = (size_t)gridDim.x * 256;
+    size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    for (; i + 3 * stride < nvec; i += 4 * stride) {
+        uint4 r[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) r[k] = __ldg(w4 + i + k * stride);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) extrema_add16<T, ASYM>(e, r[k]);
+    }
+    for (; i < nvec; i += stride) extrema_add16<T, ASYM>(e, __ldg(w4 + i));
+    for (size_t j = nvec * EPV + (size_t)blockIdx.x * 256 + threadIdx.x; j < n; j += (size_t)gridDim.x * 256)
+        extrema_add<ASYM>(e, storage_to_f32(w[j]));
+    extrema_group<256, ASYM>(e, threadIdx.x);
+    if (threadIdx.x == 0) {
+        g->partials[blockIdx.x] = e;
+        __threadfence();
+        s_last = atomicInc(arrived, gridDim.x - 1) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    e = extrema_none<ASYM>();
+    for (unsigned int k = threadIdx.x; k < gridDim.x; k += 256) {
+        const float2 o = __ldcg(reinterpret_cast<const float2 *>(g->partials + k));
+        extrema_merge<ASYM>(e, Extrema{o.x, o.y});
+    }
+    extrema_group<256, ASYM>(e, threadIdx.x);
+    if (threadIdx.x == 0) {
+        const GroupParams p = group_of<ASYM>(e, n, bits);
+        g->p = p;
+        g->f = fast_of<ASYM>(e, bits, p.zp);
+        scales[0] = p.scale;
+        if (zps) zps[0] = p.zp;
+    }
+}
+
+// U vectors per thread, requested before the wait for the first launch (which does not write them); a block covers
+// 256 * U consecutive vectors.
+template <typename T, bool ASYM, int U>
+__global__ void __launch_bounds__(256)
+quantize_tensor_kernel(const T *__restrict__ w, size_t n, const TensorGroup *g, int8_t *__restrict__ q) {
+    pdl_launch_dependents();
+    constexpr int EPV = Vec16<T>::kElems;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(w) & 15) == 0) && ((reinterpret_cast<uintptr_t>(q) & (EPV - 1)) == 0);
+    const size_t nvec = aligned ? n / EPV : 0;
+    const size_t first = (size_t)(gridDim.x - 1 - blockIdx.x) * (256 * U) + threadIdx.x;
+    const uint4 *w4 = reinterpret_cast<const uint4 *>(w);
+    uint4 r[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) r[u] = first + u * 256 < nvec ? __ldcs(w4 + first + u * 256) : make_uint4(0, 0, 0, 0);
+    pdl_wait();
+    const FastGroup f = g->f;
+    const uint32_t all = f.exact ? (1u << EPV) - 1u : 0u;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const size_t at = first + u * 256;
+        if (at >= nvec) break;
+        float x[EPV];
+        uint32_t word[EPV / 4];
+        unpack16(r[u], static_cast<const T *>(nullptr), x);
+        const uint32_t redo = quant_words<ASYM, EPV>(x, f, word) | all;
+        store_codes<EPV>(q, at, word);
+#pragma unroll 1
+        for (uint32_t left = redo; left != 0; left &= left - 1) {
+            const size_t j = at * EPV + lowest_bit(left);
+            q[j] = (int8_t)quant_ex(widen(w[j]), g->p);
+        }
+    }
+    for (size_t j = nvec * EPV + (size_t)blockIdx.x * 256 + threadIdx.x; j < n; j += (size_t)gridDim.x * 256) {
+        uint32_t m;
+        const float d = quant_candidate<ASYM>(storage_to_f32(w[j]), f, m);
+        q[j] = all || undecided<ASYM>(d) ? (int8_t)quant_ex(widen(w[j]), g->p) : (int8_t)m;
+    }
+}
+#endif  // SHREWQ_CPU_EMU
+
 struct TensorParams {
     RowParams p;
 };
@@ -263,40 +437,126 @@ __device__ __forceinline__ uint16_t f64_to_bf16_rne(double v) {
     return (uint16_t)(rounded >> 16);
 }
 
+// A code as f64 without the conversion pipe: the byte goes into the mantissa of 2^52 (u = q + 128), one subtraction leaves q.
+__device__ __forceinline__ double code_f64(uint32_t biased_byte) {
+    return __longlong_as_double((long long)(0x4330000000000000ull | biased_byte)) - 4503599627370624.0;  // 2^52 + 128
+}
+
+// Four codes of one scale -> four bf16.  The f32 product is off by less than 2 ulp of f32 and decides the rounding unless its
+// low half lies within 8 of the midpoint 0x8000; a word with such an element, and every word under a scale that is
+// not an ordinary f32 number, takes the f64 products and the sticky rounding.  Two elements at a time: the test adds 8 to
+// both low halves and looks for a half that became 0x800? (a carry out of the lower half moves the upper one by 1, well
+// inside the margin).  About 40 instructions a word against 90 with the elements one by one.
+__device__ __forceinline__ unsigned long long dq4_bf16(uint32_t biased, double s) {
+    const float f = (float)s;
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(__byte_perm(biased, 0x4B000000u, 0x7440 + j));  // 2^23 + q + 128
+    add_f32x2(v[0], v[1], -8388736.0f, -8388736.0f);
+    add_f32x2(v[2], v[3], -8388736.0f, -8388736.0f);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] *= f;
+    uint32_t near = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j += 2) {
+        const uint32_t low = __byte_perm(__float_as_uint(v[j]), __float_as_uint(v[j + 1]), 0x5410);
+        const uint32_t h = ((low + 0x00080008u) & 0xFFF0FFF0u) ^ 0x80008000u;  // a zero half: near
+        near |= (h - 0x00010001u) & ~h & 0x80008000u;
+    }
+    uint32_t lo = pack_bf16x2_rn(v[1], v[0]), hi = pack_bf16x2_rn(v[3], v[2]);
+    if (near != 0 || !(f > 1e-30f && f < 1e30f)) {
+        uint32_t h[2] = {0, 0};
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t x = (uint32_t)f64_to_bf16_rne(code_f64((biased >> (8 * j)) & 0xFFu) * s) << (16 * (j & 1));
+            if (j < 2) h[0] |= x;
+            else h[1] |= x;
+        }
+        lo = h[0];
+        hi = h[1];
+    }
+    return (unsigned long long)lo | ((unsigned long long)hi << 32);
+}
+
+// vec_ok: q is 4-byte and out 16-byte (f32) or 8-byte aligned.  A block takes 256 * U consecutive words of four codes at a
+// time, U per thread with their loads in flight together, in flat order whatever the row length (a word may straddle
+// rows).  The row of a word comes from 32-bit divisions where the tensor allows (a 64-bit division per word was a third
+// of the instructions).  Blocks of consecutive words, as many as there are, rather than a grid that strides over the
+// tensor: the stores of a block then fill whole DRAM pages.
+template <typename OutT>
+struct DequantWords {
+    static constexpr int kPerThread = sizeof(OutT) == 4 ? 4 : 8;
+};
 template <typename OutT>
 __global__ void __launch_bounds__(256)
 dequantize_kernel(const int8_t *__restrict__ q, const double *__restrict__ scales, size_t rows,
                   size_t cols, int per_channel, OutT *__restrict__ out, int vec_ok) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t n = rows * cols;
-    const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t nthreads = (size_t)gridDim.x * blockDim.x;
-    if (vec_ok) {  // cols % 4 == 0 and aligned pointers: a 4-code word never straddles a row
+    size_t done = 0;
+    if (vec_ok && (!per_channel || cols >= 4)) {
+        constexpr int U = DequantWords<OutT>::kPerThread;
         const size_t nvec = n >> 2;
+        done = nvec << 2;
         const uint32_t *q4 = reinterpret_cast<const uint32_t *>(q);
-        for (size_t i = tid; i < nvec; i += nthreads) {
-            const uint32_t wd = __ldcs(q4 + i);
-            const double s = per_channel ? __ldg(scales + (i << 2) / cols) : __ldg(scales);
-            const int a = (int)(int8_t)(wd & 0xFF), b = (int)(int8_t)((wd >> 8) & 0xFF),
-                      c = (int)(int8_t)((wd >> 16) & 0xFF), d = (int)(int8_t)(wd >> 24);
-            if constexpr (sizeof(OutT) == 4) {
-                __stcs(reinterpret_cast<float4 *>(out) + i,
-                       make_float4(dq_f32(a, s), dq_f32(b, s), dq_f32(c, s), dq_f32(d, s)));
-            } else {
-                uint2 o;
-                o.x = (uint32_t)f64_to_bf16_rne((double)a * s) | ((uint32_t)f64_to_bf16_rne((double)b * s) << 16);
-                o.y = (uint32_t)f64_to_bf16_rne((double)c * s) | ((uint32_t)f64_to_bf16_rne((double)d * s) << 16);
-                __stcs(reinterpret_cast<uint2 *>(out) + i, o);
+        const uint32_t width = per_channel ? (uint32_t)(cols < 0xFFFFFFFFull ? cols : 0xFFFFFFFFull) : 0xFFFFFFFFu;
+        const uint32_t drow = 1024u / width, dcol = 1024u - drow * width;
+        for (size_t first = (size_t)blockIdx.x * (256 * U) + threadIdx.x; first < nvec; first += (size_t)gridDim.x * (256 * U)) {
+            uint32_t b[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) b[u] = first + u * 256 < nvec ? __ldcs(q4 + first + u * 256) ^ 0x80808080u : 0u;
+            size_t row = 0, col = 0;
+            if (per_channel) {
+                const size_t e = first << 2;
+                if (n <= 0xFFFFFFFFull) {
+                    row = (uint32_t)e / width;
+                    col = (uint32_t)e - (uint32_t)row * width;
+                } else {
+                    row = e / cols;
+                    col = e - row * cols;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const size_t i = first + u * 256;
+                if (i >= nvec) break;
+                const double s0 = __ldg(scales + row);
+                if (per_channel && cols - col < 4) {
+                    // the elements of this word beyond the row's end belong to the next row
+                    const int split = (int)(cols - col);
+                    const double s1 = __ldg(scales + row + 1);
+#pragma unroll 1
+                    for (int j = 0; j < 4; ++j) {
+                        const double v = code_f64((b[u] >> (8 * j)) & 0xFFu) * (split > j ? s0 : s1);
+                        if constexpr (sizeof(OutT) == 4) out[4 * i + j] = (float)v;
+                        else out[4 * i + j] = f64_to_bf16_rne(v);
+                    }
+                } else if constexpr (sizeof(OutT) == 4) {
+                    __stcs(reinterpret_cast<float4 *>(out) + i,
+                           make_float4((float)(code_f64(b[u] & 0xFFu) * s0), (float)(code_f64((b[u] >> 8) & 0xFFu) * s0),
+                                       (float)(code_f64((b[u] >> 16) & 0xFFu) * s0), (float)(code_f64(b[u] >> 24) * s0)));
+                } else {
+                    __stcs(reinterpret_cast<unsigned long long *>(out) + i, dq4_bf16(b[u], s0));
+                }
+                if (per_channel) {
+                    row += drow;
+                    col += dcol;
+                    if (col >= cols) {
+                        col -= cols;
+                        row += 1;
+                    }
+                }
             }
         }
-    } else {
-        for (size_t i = tid; i < n; i += nthreads) {
-            const double s = per_channel ? scales[i / cols] : scales[0];
-            const int v = (int)q[i];
-            if constexpr (sizeof(OutT) == 4)
-                out[i] = dq_f32(v, s);
-            else
-                out[i] = f64_to_bf16_rne((double)v * s);
-        }
+    }
+    for (size_t i = done + (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
+        const double s = per_channel ? scales[i / cols] : scales[0];
+        const int v = (int)q[i];
+        if constexpr (sizeof(OutT) == 4)
+            out[i] = dq_f32(v, s);
+        else
+            out[i] = f64_to_bf16_rne((double)v * s);
     }
 }
 

@@ -3,6 +3,7 @@
 #include "common.cuh"
 #include <cuda_fp16.h>
 
+#include "quantize_launch.cuh"
 #include "quantize_modes_kernels.cuh"
 
 namespace shrewq {
@@ -45,6 +46,9 @@ int quantize_any_t(shrewq_ctx *ctx, const T *w, size_t rows, size_t cols, int gr
 // w_dtype: SHREWQ_F32, SHREWQ_BF16, SHREWQ_F16 or SHREWQ_F64 (the storage type of the tensor)
 int launch_quantize_any(shrewq_ctx *ctx, const void *w, int w_dtype, size_t rows, size_t cols, int granularity, int bits,
                         int mode, int8_t *q, double *scales, double *zps) {
+    bool taken = false;
+    int rc = launch_quantize_tuned(ctx, w, w_dtype, rows, cols, granularity, bits, mode, q, scales, zps, &taken);
+    if (rc != SHREWQ_OK || taken) return rc;
     switch (w_dtype) {
         case SHREWQ_F32: return quantize_any_t(ctx, static_cast<const float *>(w), rows, cols, granularity, bits, mode, q, scales, zps);
         case SHREWQ_BF16: return quantize_any_t(ctx, static_cast<const __nv_bfloat16 *>(w), rows, cols, granularity, bits, mode, q, scales, zps);
@@ -56,7 +60,7 @@ int launch_quantize_any(shrewq_ctx *ctx, const void *w, int w_dtype, size_t rows
 
 int launch_quantize_ex(shrewq_ctx *ctx, const float *w, size_t rows, size_t cols, int granularity, int bits, int mode,
                        int8_t *q, double *scales, double *zps) {
-    return quantize_any_t(ctx, w, rows, cols, granularity, bits, mode, q, scales, zps);
+    return launch_quantize_any(ctx, w, SHREWQ_F32, rows, cols, granularity, bits, mode, q, scales, zps);
 }
 
 // zps may be null (zero points of 0.0); out_dtype: SHREWQ_F32, SHREWQ_BF16, SHREWQ_F16 or SHREWQ_F64

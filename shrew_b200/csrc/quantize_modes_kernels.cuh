@@ -1,16 +1,6 @@
-// Quantize / dequantize in the reference's other modes: asymmetric INT8, INT4 symmetric and
-// asymmetric (one code per byte, as the reference stores them), sm_100a.
-//
-// Reference semantics (crates/shrew/src/quantize.rs), all in f64 on a widened copy:
-//   qmax = 127 | 7;  qmin = -127 | -7 (symmetric), -128 | -8 (asymmetric)          (:124-139)
-//   symmetric : scale = amax < 1e-30 ? 1 : amax / qmax,  zp = 0                     (:349-352)
-//   asymmetric: range = max - min;  scale = range < 1e-30 ? 1 : range / (qmax - qmin);
-//               zp = round(qmin - min / scale)                                      (:353-364)
-//   inv  = |scale| < 1e-30 ? 0 : 1 / scale                                          (:236-240)
-//   code = clamp(round_half_away(v * inv + zp), qmin, qmax) as i8   (NaN -> 0)      (:244-250)
-//   back = (code - zp) * scale                                                      (:262-266)
-// Correctness first: the element map runs the reference's f64 operations one for one (no f32
-// shortcut as in the INT8 symmetric kernels); min, max and amax of f32 values are exact in f32.
+// Quantize / dequantize in every mode and storage type, one f64 operation for one of the reference's, sm_100a: what the
+// tuned kernels (quantize_kernels.cuh) do not take (f64 tensors, rows too long for registers), and dequantize with zero
+// points or to f16 / f64.  The arithmetic: quantize_common.cuh.
 // Per-channel rows are read twice (the second pass normally from L2); per-tensor takes three
 // launches (min/max with atomics on order-preserving integer keys, parameters, element map).
 //
@@ -19,66 +9,10 @@
 // thread and compare them with the golden vectors (tests/cpu_emu/).
 #pragma once
 
-#include "../../include/shrewq.h"
-#ifndef SHREWQ_CPU_EMU
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
-#include <cuda_runtime.h>
-#include <stdint.h>
-#endif
+#include "quantize_common.cuh"
 
 namespace shrewq {
 namespace {
-
-struct GroupParams {
-    double scale, zp, inv, qmin, qmax;
-};
-
-__device__ __forceinline__ double qmax_of(int bits) { return bits == 4 ? 7.0 : 127.0; }
-__device__ __forceinline__ double qmin_of(int bits, int mode) {
-    if (bits == 4) return mode == SHREWQ_ASYMMETRIC ? -8.0 : -7.0;
-    return mode == SHREWQ_ASYMMETRIC ? -128.0 : -127.0;
-}
-
-__device__ __forceinline__ double round_half_away(double t) {
-    if (t != t) return t;
-    double r = trunc(t);
-    if (fabs(t - r) >= 0.5) r += copysign(1.0, t);  // t - r is exact; false for +-Inf (NaN compare)
-    return copysign(r, t);                          // round(-0.3) is -0.0, as f64::round
-}
-
-// Tensor element -> f64, exactly (Tensor::to_f64_vec, quantize.rs:198): f32, f64, bf16 or f16 storage.
-__device__ __forceinline__ double widen(float v) { return (double)v; }
-__device__ __forceinline__ double widen(double v) { return v; }
-__device__ __forceinline__ double widen(__nv_bfloat16 v) { return (double)__bfloat162float(v); }
-__device__ __forceinline__ double widen(__half v) { return (double)__half2float(v); }
-
-// compute_scale_zp for a group of n elements whose extrema are lo / hi / amax (f64: exact for every
-// storage type)
-__device__ __forceinline__ GroupParams make_group(double lo, double hi, double amax, size_t n, int bits, int mode) {
-    GroupParams p;
-    p.qmin = qmin_of(bits, mode);
-    p.qmax = qmax_of(bits);
-    if (n == 0) {
-        p.scale = 1.0;
-        p.zp = 0.0;
-    } else if (mode != SHREWQ_ASYMMETRIC) {
-        p.scale = amax < 1e-30 ? 1.0 : amax / p.qmax;
-        p.zp = 0.0;
-    } else {
-        const double range = hi - lo;
-        p.scale = range < 1e-30 ? 1.0 : range / (p.qmax - p.qmin);
-        p.zp = round_half_away(p.qmin - lo / p.scale);
-    }
-    p.inv = fabs(p.scale) < 1e-30 ? 0.0 : 1.0 / p.scale;
-    return p;
-}
-
-__device__ __forceinline__ int quant_ex(double v, const GroupParams &p) {
-    const double t = round_half_away(__dadd_rn(__dmul_rn(v, p.inv), p.zp));
-    if (t != t) return 0;  // NaN as i8 == 0
-    return (int)fmin(fmax(t, p.qmin), p.qmax);
-}
 
 __device__ __forceinline__ double warp_min(double v) {
 #pragma unroll
