@@ -170,7 +170,7 @@ linear_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const 
         // Programmatic dependent launch: the WEIGHTS of the first stages are requested at once (they never depend on
         // an earlier kernel), the activations only when the previous kernel of the stream, whose output they may be,
         // has completed (griddepcontrol.wait; it returns at once in an ordinary launch).
-        if (lane == 0) {
+        if (elect_one()) {
             auto load_w = [&](uint32_t dst, int kc, uint32_t wb) {
 #pragma unroll
                 for (int j = 0; j < kSub; ++j) {
@@ -218,7 +218,7 @@ linear_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const 
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (one thread of the leader CTA) ----------------
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             // D=f32, A=bf16 (K-major, TMEM), B=bf16 (K-major), M=256 (two CTAs), N=256
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTokPair >> 3) << 17) |
                                        ((uint32_t)((2 * kLanes) >> 4) << 24);

@@ -168,7 +168,7 @@ linear_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
         // Programmatic dependent launch: the WEIGHTS of the first stages are requested at once (they never depend on
         // an earlier kernel), the activations only when the previous kernel of the stream, whose output they may be,
         // has completed (griddepcontrol.wait; it returns at once in an ordinary launch).
-        if (lane == 0) {
+        if (elect_one()) {
             auto load_w = [&](uint32_t dst, int kc, uint32_t fb) {
 #pragma unroll
                 for (int j = 0; j < KSUB; ++j) {
@@ -219,7 +219,7 @@ linear_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (one thread) ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             // instruction descriptor: D=f32, A=bf16 (K-major, from TMEM), B=bf16 (K-major), M=128, N=TOK
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
                                        ((uint32_t)(TOK >> 3) << 17) | ((uint32_t)(kTileN >> 4) << 24);

@@ -43,6 +43,7 @@
 #include "../../include/shrewq.h"
 #include "dests.cuh"
 #include "ptx_small.cuh"
+#include "widen_bf16.cuh"
 #include "activation_f16.cuh"
 
 namespace shrewq {
@@ -51,17 +52,6 @@ namespace {
 constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
 constexpr int NB = 2;  // channel blocks of 8 per warp
-
-// 4 INT8 codes -> two packed bf16x2 words, exactly (see gemm_tcgen05.cu for the trick)
-__device__ __forceinline__ void cvt_i8x4_bf16(uint32_t w, uint32_t &lo, uint32_t &hi) {
-    const uint32_t u = w ^ 0x80808080u;
-    const float f0 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7440)) - 8388736.0f;
-    const float f1 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7441)) - 8388736.0f;
-    const float f2 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7442)) - 8388736.0f;
-    const float f3 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7443)) - 8388736.0f;
-    lo = pack_bf16x2_rn(f1, f0);
-    hi = pack_bf16x2_rn(f3, f2);
-}
 
 // 4 INT8 codes -> two packed f16x2 words, exactly: (1024 + (code + 128)) - 1152
 __device__ __forceinline__ void cvt_i8x4_f16(uint32_t w, uint32_t &lo, uint32_t &hi) {

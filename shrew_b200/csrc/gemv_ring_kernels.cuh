@@ -41,6 +41,7 @@
 #include "dests.cuh"
 #include "ptx_small.cuh"
 #include "ptx_tcgen05.cuh"
+#include "widen_bf16.cuh"
 
 namespace shrewq {
 namespace {
@@ -66,20 +67,6 @@ struct RingCfg {
 };
 constexpr int kRingKC = 2048;     // what the launcher instantiates
 constexpr int kRingConsumers = 8;
-
-// 4 INT8 codes (one word) -> two packed bf16x2 words, exactly: byte ^ 0x80 = q + 128 as an unsigned byte u;
-// 0x4B0000uu is the float 2^23 + u; subtracting 2^23 + 128 leaves q; the pack is exact for |q| <= 128
-__device__ __forceinline__ void ring_cvt_i8x4(uint32_t w, uint32_t &lo, uint32_t &hi) {
-    const uint32_t u = w ^ 0x80808080u;
-    float f0 = __uint_as_float((u & 0xFFu) | 0x4B000000u);                 // one logic op; the others a byte permute
-    float f1 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7441));
-    float f2 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7442));
-    float f3 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7443));
-    add_f32x2(f0, f1, -8388736.0f, -8388736.0f);
-    add_f32x2(f2, f3, -8388736.0f, -8388736.0f);
-    lo = pack_bf16x2_rn(f1, f0);
-    hi = pack_bf16x2_rn(f3, f2);
-}
 
 template <typename YT>
 __device__ __forceinline__ void ring_store(YT *p, float v);
@@ -214,8 +201,8 @@ gemv_i8_ring_kernel(const int8_t *__restrict__ q, const float *__restrict__ scal
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 uint32_t a0, a1, a2, a3;
-                ring_cvt_i8x4(wl[j], a0, a2);  // row g:     codes (4j, 4j+1) | (4j+2, 4j+3)
-                ring_cvt_i8x4(wh[j], a1, a3);  // row g + 8
+                cvt_i8x4_bf16(wl[j], a0, a2);  // row g:     codes (4j, 4j+1) | (4j+2, 4j+3)
+                cvt_i8x4_bf16(wh[j], a1, a3);  // row g + 8
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
                     const uint4 &xa = xc[nt][j >> 1];

@@ -11,6 +11,14 @@
 namespace shrewq {
 namespace {
 
+// true in exactly one lane of a converged warp; unlike a comparison of the lane number it tells the compiler that a single
+// thread is inside the branch, where the instructions with warp-uniform operands (tcgen05.mma, TMA) stand
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {

@@ -5,6 +5,7 @@
 #include "dests.cuh"
 #include "ptx_small.cuh"
 #include "ptx_tcgen05.cuh"
+#include "widen_bf16.cuh"
 
 namespace shrewq {
 namespace {
@@ -70,19 +71,6 @@ __device__ __forceinline__ bool mbar_wait_warp_c(uint32_t bar, uint32_t parity, 
     // each has its own acquire on the data the barrier guards
     if (ok) ok = mbar_try(bar, parity) ? 1 : 0;
     return __all_sync(0xFFFFFFFFu, ok) != 0;
-}
-
-// 4 INT8 codes (one 32-bit word) -> two packed bf16x2 words, exactly.
-// byte ^ 0x80 = q + 128 as an unsigned byte u; 0x4B0000uu is the float 2^23 + u; subtracting
-// 2^23 + 128 leaves q; cvt.rn.bf16x2.f32 packs two of them (exact, |q| <= 128).
-__device__ __forceinline__ void cvt_i8x4_bf16(uint32_t w, uint32_t &lo, uint32_t &hi) {
-    const uint32_t u = w ^ 0x80808080u;
-    const float f0 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7440)) - 8388736.0f;
-    const float f1 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7441)) - 8388736.0f;
-    const float f2 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7442)) - 8388736.0f;
-    const float f3 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7443)) - 8388736.0f;
-    lo = pack_bf16x2_rn(f1, f0);
-    hi = pack_bf16x2_rn(f3, f2);
 }
 
 // One weight row's 64 codes of a 64-byte-swizzled INT8 sub-block -> 32 packed bf16x2 words.  TMA wrote the

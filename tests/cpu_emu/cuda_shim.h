@@ -299,6 +299,16 @@ static inline void add_f32x2(float &a0, float &a1, float b0, float b1) { a0 += b
 static inline uint32_t pack_bf16x2_rn(float hi, float lo) {
     return ((uint32_t)__float2bfloat16_rn(hi).bits << 16) | __float2bfloat16_rn(lo).bits;
 }
+static inline float emu_f32_of_bf16(uint32_t bits16) { uint32_t u = bits16 << 16; float f; memcpy(&f, &u, 4); return f; }
+// (the products and sums the kernels form here are exact in f32, so one rounding to bf16 is the fused result)
+static inline uint32_t fma_bf16x2(uint32_t a, uint32_t b, uint32_t c) {
+    return pack_bf16x2_rn(emu_f32_of_bf16(a >> 16) * emu_f32_of_bf16(b >> 16) + emu_f32_of_bf16(c >> 16),
+                          emu_f32_of_bf16(a & 0xFFFF) * emu_f32_of_bf16(b & 0xFFFF) + emu_f32_of_bf16(c & 0xFFFF));
+}
+static inline uint32_t fma_relu_bf16x2(uint32_t a, uint32_t b, uint32_t c) {
+    const uint32_t d = fma_bf16x2(a, b, c);
+    return ((d & 0x80000000u) ? 0u : d & 0xFFFF0000u) | ((d & 0x8000u) ? 0u : d & 0xFFFFu);
+}
 static inline _Float16 emu_f16_of(uint32_t bits16) { uint16_t u = (uint16_t)bits16; _Float16 h; memcpy(&h, &u, 2); return h; }
 static inline uint32_t emu_bits_of(_Float16 h) { uint16_t u; memcpy(&u, &h, 2); return u; }
 static inline uint32_t sub_f16x2(uint32_t a, uint32_t b) {

@@ -68,6 +68,8 @@ inline void mbar_settle(MBar *b) {
 }
 }  // namespace emu
 
+// the elected lane of a converged warp: lane 0 here
+static inline bool elect_one() { return (threadIdx.x & 31u) == 0; }
 static inline uint32_t smem_u32(const void *p) { return (uint32_t)reinterpret_cast<uintptr_t>(p); }
 
 static inline void mbar_init(uint32_t bar, uint32_t count) {
