@@ -96,6 +96,8 @@ SHREWQ_API int shrewq_ctx_set_stream(shrewq_ctx *ctx, void *stream);
  *                         kernel does so for tails of up to a quarter wave, 1 = whenever a tail exists, 2 = never
  *   "tc_pair"      0..2   CTA pairs (tcgen05.mma.cta_group::2) for batches above 128 tokens: 0 never, 1 where
  *                         they win by measurement (default), 2 always
+ *   "tc_f32"       0..2   the persistent kernel for f32 activations and outputs: 0 never, 1 where it wins by
+ *                         measurement (default), 2 whenever it can take the call
  *   "ring_stages"  0, 2, 3  stages of the ring kernel's shared-memory ring (default 0 = three while all its CTAs are
  *                         resident at once, two for larger grids)
  *   "pdl"          0/1    programmatic dependent launch of the forward kernels (default 1): from a handle's second

@@ -19,7 +19,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libshrewq.so")
 HOST_EXT = os.path.join(HERE, "_host.so")
-SOURCES = ["api.cu", "quantize.cu", "quantize_batch.cu", "quantize_modes.cu", "gemv.cu", "gemv_mma.cu", "gemm_simt.cu", "gemm_tcgen05.cu", "gemm_tcgen05_g1.cu", "gemm_tcgen05_g2.cu", "gemm_tcgen05_g3.cu", "gemm_tcgen05_2cta.cu", "exchange.cu"]
+SOURCES = ["api.cu", "quantize.cu", "quantize_batch.cu", "quantize_modes.cu", "gemv.cu", "gemv_mma.cu", "gemm_simt.cu", "gemm_tcgen05.cu", "gemm_tcgen05_g1.cu", "gemm_tcgen05_g2.cu", "gemm_tcgen05_g3.cu", "gemm_tcgen05_2cta.cu", "gemm_tcgen05_f32.cu", "exchange.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
          "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]

@@ -146,6 +146,10 @@ int shrewq_ctx_set_option(shrewq_ctx *ctx, const char *name, int value) {
         t.tc_pair = value;
     }
     else if (!strcmp(name, "pdl") || !strcmp(name, "gemv_pdl")) t.pdl = value != 0;
+    else if (!strcmp(name, "tc_f32")) {
+        if (value < 0 || value > 2) return set_err(ctx, SHREWQ_ERR_INVALID_ARG, "set_option: tc_f32 is 0 (never), 1 (where it wins) or 2 (whenever it can)");
+        t.tc_f32 = value;
+    }
     else if (!strcmp(name, "ring_stages")) t.ring_stages = value == 2 || value == 3 ? value : 0;
     else return set_err(ctx, SHREWQ_ERR_INVALID_ARG, "set_option: unknown option '%s'", name);
     return SHREWQ_OK;
@@ -561,6 +565,7 @@ const char *shrewq_linear_last_kernel(const shrewq_linear *lin) { return lin ? g
 // accumulator, so the codes are read and converted once and the result keeps the f32 path's 1e-4 tolerance.
 static int forward_f32_on_tensor_cores(shrewq_linear *lin, const ForwardArgs &orig, const char *who) {
     shrewq_ctx *ctx = lin->ctx;
+    if (tcgen05_f32_wins(orig, ctx->tuning)) return launch_gemm_tcgen05_f32(ctx, orig, lin->w_tmap);
     const size_t n = orig.M * orig.K;
     int rc = ensure_xsplit(ctx, 2 * n * 2);
     if (rc != SHREWQ_OK) return rc;

@@ -26,6 +26,7 @@ struct Tuning {
     int tc_tok_gated = 0;   // the same for gate/up launches only
     int tc_tailsplit = 0;   // a short last wave as a second launch split along K: 0 = pair kernel, tails up to a quarter wave; 1 = always; 2 = never
     int tc_pair = 1;        // CTA pairs (tcgen05.mma.cta_group::2) for large batches: 0 never, 1 where they win, 2 whenever M > 128
+    int tc_f32 = 1;         // persistent kernel for f32 activations: 0 never, 1 where it wins, 2 whenever it can
     int ring_stages = 0;    // stages of the ring kernel: 0 = by grid size, 2 or 3 forced
     int pdl = 1;            // programmatic dependent launch of the forward kernels (after a handle's first forward)
 };
@@ -176,6 +177,8 @@ int plan_gemm_tcgen05(size_t M, size_t N, size_t K, bool gated, int sm_count, in
                       int *splits, int *rounds_per_split);
 int launch_gemm_tcgen05_2cta(shrewq_ctx *ctx, const ForwardArgs &a, const void *w_tmap, const void *w_up_tmap);
 int launch_gemm_tcgen05_noalloc(shrewq_ctx *ctx, const ForwardArgs &a, const void *w_tmap);
+bool tcgen05_f32_wins(const ForwardArgs &a, const Tuning &t);
+int launch_gemm_tcgen05_f32(shrewq_ctx *ctx, const ForwardArgs &a, const void *w_tmap);
 int launch_gemm_tcgen05_xsplit(shrewq_ctx *ctx, const ForwardArgs &a, const void *w_tmap);
 int encode_weight_tmap(shrewq_ctx *ctx, const int8_t *q, size_t n, size_t k, int box_rows, void *tmap_out);
 

@@ -57,6 +57,9 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void *src, uint
                  : "memory");
 }
 
+// this thread's writes to shared memory become visible to the async proxy (tcgen05.mma operands, TMA stores)
+__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 

@@ -216,6 +216,7 @@ inline void tc_progress() {
 }
 }  // namespace emu
 
+static inline void fence_proxy_async_smem() {}
 static inline void tc_fence_before() {}
 static inline void tc_fence_after() {}
 static inline void tc_wait_st() {}

@@ -663,6 +663,53 @@ def test_f32_activations_as_hi_lo_pair_on_the_tensor_cores(oracle, emu, emu_tc, 
     assert oracle.rel_err(got, ref) < (1e-2 if y_bf16 else 1e-4)   # the f32 path's tolerance
 
 
+# The persistent f32-activation kernel: one to three CTAs share the tiles, so that a CTA crosses token tiles, reuses both
+# accumulators and wraps every ring; K on both sides of what stays resident (768 features with 64-token tiles, 384 with
+# 128); ragged M, N, K and output rows off 16 bytes.  `late`: copies and MMAs complete late and out of order.
+# Bound: the split keeps x to 2^-17 of each value (hi and lo rounded to nearest, 8 significant bits each), the sums are
+# f32, so the relative error stays below 2^-16 + K * 2^-24 of sum |q||x|, with non-negative x below 1e-4 of the result's norm.
+@pytest.mark.parametrize("tok,M,N,K,ldy,ctas,late", [
+    (64, 64, 128, 16, 128, 1, 0), (64, 65, 129, 80, 131, 1, 0), (64, 130, 300, 256, 300, 2, 3), (64, 200, 520, 768, 521, 3, 0),
+    (64, 70, 130, 784, 130, 1, 5), (64, 100, 200, 1024, 200, 3, 0), (128, 128, 128, 64, 128, 1, 0), (128, 129, 257, 256, 257, 2, 7),
+    (128, 300, 300, 384, 301, 1, 0), (128, 130, 140, 400, 140, 2, 0)])
+def test_tcgen05_persistent_f32_forward(oracle, tok, M, N, K, ldy, ctas, late):
+    L = _build("emu_gemm_tcgen05_f32")
+    L.emu_gemm_tcgen05_f32.argtypes = [_vp, _vp, _vp, _vp, _vp, _ci, _ci, _ci, _sz, _ci, _ci, _ci]
+    L.emu_fail_message.restype = ctypes.c_char_p
+    rng = np.random.default_rng(M + N + K)
+    q = _aligned((N, K), np.int8)
+    q[...] = rng.integers(-128, 128, size=(N, K)).astype(np.int8)
+    scales = rng.random(N) * 1e-2 + 1e-4
+    bias = (rng.standard_normal(N) * 0.1).astype(np.float32)
+    x = _aligned((M, K), np.float32)
+    x[...] = rng.random((M, K))
+    relu = (M + N) % 2
+    y = np.full((M, ldy), 7.0, np.float32)
+    s32 = scales.astype(np.float32)
+    L.emu_tma_async(late, 4)
+    try:
+        rc = L.emu_gemm_tcgen05_f32(_p(q), _p(s32), _p(bias), _p(x), _p(y), M, N, K, ldy, relu, tok, ctas)
+    finally:
+        L.emu_tma_async(0, 8)
+    assert rc == 0, L.emu_fail_message()
+    ref = oracle.np_linear_forward(q, scales, oracle.PER_CHANNEL, bias, x, relu=bool(relu))
+    assert oracle.rel_err(y[:, :N], ref) < 1e-4
+    assert np.all(y[:, N:] == 7.0)
+
+
+def test_tcgen05_persistent_f32_forward_ends_when_a_load_never_lands():
+    L = _build_short_waits("emu_gemm_tcgen05_f32")
+    L.emu_gemm_tcgen05_f32.argtypes = [_vp, _vp, _vp, _vp, _vp, _ci, _ci, _ci, _sz, _ci, _ci, _ci]
+    q, x = _aligned((300, 256), np.int8), _aligned((100, 256), np.float32)
+    q[...], x[...] = 1, 1.0
+    s32, y = np.ones(300, np.float32), np.zeros((100, 300), np.float32)
+    try:
+        L.emu_drop_tma(5)
+        assert L.emu_gemm_tcgen05_f32(_p(q), _p(s32), None, _p(x), _p(y), 100, 300, 256, 300, 0, 64, 2) == -2
+    finally:
+        L.emu_drop_tma(-1)
+
+
 # ---- the CTA-pair kernel (cta_group::2): two blocks of a cluster run concurrently over modelled cluster
 # shared memory.  The cta_group::2 parts of the model (tests/cpu_emu/cuda_shim_tcgen05_pair.h) state how the
 # documentation is read here; the kernel's GPU parity tests have since confirmed that reading.
