@@ -217,6 +217,12 @@ static bool ring_kernel_wins(size_t M, size_t N, bool gated, int sm_count) {
     const size_t ctas = (N + (gated ? 7 : 15)) / (gated ? 8 : 16);
     return M >= 3 && M <= 16 && ctas <= (size_t)5 * sm_count;
 }
+// Calls of the other small-batch families that the ring kernel runs faster since a CTA walks several row blocks: up to 16
+// tokens every warp-MMA call (gate/up 11008 x 4096 at 8 tokens 40.3 -> 21.3 us, 32000 x 4096 50.1 -> 30.6), and two tokens on
+// weights from 2^25 codes with bf16 results (25.6 -> 20.4 and 35.2 -> 28.0 us; at one token the GEMV stays ahead: 19.4 against 20.2 us).
+static bool ring_kernel_takes_over(int family, size_t M, size_t N, size_t K, bool gated, bool y_bf16) {
+    return (family == kForceMma && M <= 16) || (family == kForceGemv && M == 2 && y_bf16 && N * K * (gated ? 2 : 1) >= ((size_t)1 << 25));
+}
 static int default_family(size_t M, size_t N, bool gated, int sm_count, bool gemv_ok, bool mma_ok, bool tc_ok) {
     if (gemv_ok && (M <= 2 || (!mma_ok && (M <= 4 || !tc_ok)))) return kForceGemv;
     if (mma_ok && M <= 32) return ring_kernel_wins(M, N, gated, sm_count) ? kForceRing : kForceMma;
@@ -686,6 +692,7 @@ static int forward_impl(shrewq_linear *lin, shrewq_linear *up, const void *x_dev
                 choice = kForceTc2Cta;
             } else {
                 choice = default_family(M, lin->n, up != nullptr, ctx->sm_count, gemv_ok, mma_ok, tc_ok);
+                if (ring_kernel_takes_over(choice, M, lin->n, lin->k, up != nullptr, a.y_dtype == SHREWQ_BF16) && gemv_ring_supported(a)) choice = kForceRing;
             }
     }
     const char *name;

@@ -68,7 +68,8 @@ int launch_ring_stages(shrewq_ctx *ctx, const ForwardArgs &a) {
         if (d >= 0 && d < 64) attr_done.fetch_or(1ull << d, std::memory_order_release);
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((a.N + NCH - 1) / NCH));
+    const size_t blocks = (a.N + NCH - 1) / NCH, resident = (size_t)(STAGES == 2 ? 3 : 2) * ctx->sm_count;
+    cfg.gridDim = dim3((unsigned)(blocks < resident ? blocks : resident));
     cfg.blockDim = dim3((kRingConsumers + 1) * 32);
     cfg.dynamicSmemBytes = kSmem;
     cfg.stream = ctx->stream;

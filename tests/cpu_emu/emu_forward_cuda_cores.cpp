@@ -69,7 +69,8 @@ void ring_one_kc(const Args &a) {
     constexpr int NCH = GATED ? kRingRows / 2 : kRingRows;
     const unsigned grid = (unsigned)((a.N + NCH - 1) / NCH);
     if (g_ring_two_stages) {  // the launcher's choice for grids of several waves
-        emu::launch(grid, (kRingConsumers + 1) * 32, RingCfg<KC, 2>::kSmemBytes, [&] {
+        // (a third of the CTAs: each walks up to three row blocks through the ring)
+        emu::launch((grid + 2) / 3, (kRingConsumers + 1) * 32, RingCfg<KC, 2>::kSmemBytes, [&] {
             gemv_i8_ring_kernel<NT, KC, kRingConsumers, YT, GATED, 2>(a.q, a.scales, a.bias, a.q_up, a.scales_up, a.bias_up,
                                                                       static_cast<const uint16_t *>(a.x), static_cast<YT *>(a.y),
                                                                       g_peers, a.M, a.N, a.K, a.ldy, a.epilogue, &g_ring_status);
