@@ -202,7 +202,10 @@ uint64_t shrewq_ctx_launch_count(const shrewq_ctx *ctx) { return ctx ? ctx->laun
 
 // The default kernel family of a forward with bf16 activations: the one rule, shared by forward_impl and
 // shrewq_plan_forward.  Measured on 4096 x 4096, 11008 x 4096, 4096 x 11008, 1376 x 4096 and 32000 x 4096: the
-// CUDA-core GEMV wins up to 2 tokens, a warp-MMA kernel from 3 to 32, the tcgen05 kernel above.  Of the two warp-MMA
+// CUDA-core GEMV wins up to 2 tokens, a warp-MMA kernel from 3 to 16 and on small weights to 32, the tcgen05 kernel above:
+// at 24 tokens 4096 x 4096 takes 11.4 us on warp MMA and 11.1 on tcgen05, but 4096 x 11008 25.5 against 17.1 us and the
+// 11008 x 4096 gate/up pair 48.2 against 37.5 us, hence the line at 2^25 codes (bf16 results only: the
+// warps of the other kernel sum shorter chains, which an f32 result shows).  Of the two warp-MMA
 // kernels the ring kernel (bulk copies into shared memory) wins up to 16 tokens on grids of up to five CTAs per SM
 // (three stages while all CTAs are resident at once, two stages beyond: see launch_ring_one), the register-streaming
 // one on larger grids (32000 x 4096: 37 against 41 us) and above 16 tokens.
@@ -223,8 +226,10 @@ static bool ring_kernel_wins(size_t M, size_t N, bool gated, int sm_count) {
 static bool ring_kernel_takes_over(int family, size_t M, size_t N, size_t K, bool gated, bool y_bf16) {
     return (family == kForceMma && M <= 16) || (family == kForceGemv && M == 2 && y_bf16 && N * K * (gated ? 2 : 1) >= ((size_t)1 << 25));
 }
-static int default_family(size_t M, size_t N, bool gated, int sm_count, bool gemv_ok, bool mma_ok, bool tc_ok) {
+static int default_family(size_t M, size_t N, size_t K, bool gated, bool y_bf16, int sm_count, bool gemv_ok, bool mma_ok,
+                          bool tc_ok) {
     if (gemv_ok && (M <= 2 || (!mma_ok && (M <= 4 || !tc_ok)))) return kForceGemv;
+    if (mma_ok && tc_ok && y_bf16 && M > 16 && M <= 32 && N * K * (gated ? 2 : 1) >= ((size_t)1 << 25)) return kForceTc;
     if (mma_ok && M <= 32) return ring_kernel_wins(M, N, gated, sm_count) ? kForceRing : kForceMma;
     return tc_ok ? kForceTc : (gemv_ok ? kForceGemv : kForceSimt);
 }
@@ -251,7 +256,7 @@ int shrewq_plan_forward(size_t M, size_t N, size_t K, int x_is_bf16, int gated, 
     const bool small = M < (1u << 31) && N < (1u << 31) && K < (1u << 31);
     const bool tc_ok = x_is_bf16 && vec16 && M >= 1 && small;
     const bool mma_ok = x_is_bf16 && (K % 64) == 0 && M <= 64 && small;
-    int fam = default_family(M, N, gated != 0, sm_count, vec16 && M <= 16, mma_ok, tc_ok);
+    int fam = default_family(M, N, K, gated != 0, true, sm_count, vec16 && M <= 16, mma_ok, tc_ok);
     if (!x_is_bf16 && vec16 && small && M > 16 && !gated) fam = kForceTcF32;   // f32 activations: the hi/lo tensor-core pass
     if (!x_is_bf16 && vec16 && small && gemv_slices_win(M, N, K)) fam = kForceGemv;
     if (fam == kForceTc && M > 128 && pair_kernel_wins(M, N, K, gated != 0)) fam = kForceTc2Cta;
@@ -691,7 +696,7 @@ static int forward_impl(shrewq_linear *lin, shrewq_linear *up, const void *x_dev
             } else if (M > 128 && tc_ok && (ctx->tuning.tc_pair == 2 || (ctx->tuning.tc_pair == 1 && pair_kernel_wins(M, lin->n, lin->k, up != nullptr)))) {
                 choice = kForceTc2Cta;
             } else {
-                choice = default_family(M, lin->n, up != nullptr, ctx->sm_count, gemv_ok, mma_ok, tc_ok);
+                choice = default_family(M, lin->n, lin->k, up != nullptr, a.y_dtype == SHREWQ_BF16, ctx->sm_count, gemv_ok, mma_ok, tc_ok);
                 if (ring_kernel_takes_over(choice, M, lin->n, lin->k, up != nullptr, a.y_dtype == SHREWQ_BF16) && gemv_ring_supported(a)) choice = kForceRing;
             }
     }
