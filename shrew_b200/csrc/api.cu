@@ -210,8 +210,8 @@ uint64_t shrewq_ctx_launch_count(const shrewq_ctx *ctx) { return ctx ? ctx->laun
 // (three stages while all CTAs are resident at once, two stages beyond: see launch_ring_one), the register-streaming
 // one on larger grids (32000 x 4096: 37 against 41 us) and above 16 tokens.
 // f32 activations on SMALL layers (config 1: 784 -> 256 -> 10 at 64 tokens): the whole forward is a few MFLOP and
-// what counts is the number and latency of launches; the CUDA-core GEMV in slices of 16 tokens is one short launch
-// where the tensor-core route is a split pass plus a pipelined kernel that never fills.
+// what counts is the number and latency of launches; the CUDA-core GEMV in slices of tokens is one short launch
+// where the tensor-core route never fills (and it keeps every bit of x, which the hi/lo pair does not).
 constexpr size_t kGemvSlicedMaxTokens = 128;
 static bool gemv_slices_win(size_t M, size_t N, size_t K) {
     return M > 16 && M <= kGemvSlicedMaxTokens && M * N * K <= ((size_t)1 << 26);

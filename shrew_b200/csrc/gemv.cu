@@ -52,7 +52,10 @@ void dispatch_m(shrewq_ctx *ctx, const ForwardArgs &a) {
     else if (a.M <= 2) launch_one<2, 4, XT, YT, GATED>(ctx, a);
     else if (a.M <= 4) launch_one<4, 4, XT, YT, GATED>(ctx, a);
     else if (a.M <= 8) launch_one<8, 2, XT, YT, GATED>(ctx, a);
-    else launch_one<16, 2, XT, YT, GATED>(ctx, a);
+    else if (a.M <= 16) launch_one<16, 2, XT, YT, GATED>(ctx, a);
+    // slices: of 4 tokens, since a CTA's own latency is the time of these calls and 16 tokens a thread are 160 shuffles at its
+    // end: 64 x 1024 x 1024 36.1 -> 22.7 us, 40 x 512 x 768 15.4 -> 7.9, 64 x 256 x 784 12 -> 7.5
+    else launch_one<4, 4, XT, YT, GATED>(ctx, a);
 }
 
 // ---- the ring kernel (1..32 tokens, bf16 activations): bulk copies into a shared-memory ring + warp MMA ----

@@ -53,7 +53,8 @@ void gemv_m(const Args &a) {
     else if (a.M <= 2) gemv_one<2, 4, XT, YT, GATED>(a);
     else if (a.M <= 4) gemv_one<4, 4, XT, YT, GATED>(a);
     else if (a.M <= 8) gemv_one<8, 2, XT, YT, GATED>(a);
-    else gemv_one<16, 2, XT, YT, GATED>(a);
+    else if (a.M <= 16) gemv_one<16, 2, XT, YT, GATED>(a);
+    else gemv_one<4, 4, XT, YT, GATED>(a);
 }
 template <typename XT, typename YT>
 void gemv_g(const Args &a) {
