@@ -366,7 +366,8 @@ SHREWQ_API int shrewq_force_kernel(const char *name);
 /* Which kernel family and launch plan a forward of this shape would get on a GPU with `sm_count` SMs
  * (16-byte aligned buffers, no forced kernel): writes the family name into `kernel` (at least 16 bytes)
  * and, for "tcgen05", the token tile, the tile grid, the K splits and the pipeline rounds per split
- * (zeros otherwise).  Pure host arithmetic: needs no GPU and no context.  For tests, benchmarks and
+ * (zeros otherwise).  "mma" stands for both warp-MMA kernels: up to 16 tokens its calls run on the ring kernel, and two
+ * tokens of "gemv" do on large weights with bf16 results.  Pure host arithmetic: needs no GPU and no context.  For tests, benchmarks and
  * capacity planning; no counterpart in the reference. */
 SHREWQ_API int shrewq_plan_forward(size_t M, size_t N, size_t K, int x_is_bf16, int gated, int sm_count, char *kernel,
                         size_t kernel_len, int *tok, int *n_tiles, int *m_tiles, int *splits,

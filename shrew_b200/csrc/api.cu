@@ -206,9 +206,9 @@ uint64_t shrewq_ctx_launch_count(const shrewq_ctx *ctx) { return ctx ? ctx->laun
 // at 24 tokens 4096 x 4096 takes 11.4 us on warp MMA and 11.1 on tcgen05, but 4096 x 11008 25.5 against 17.1 us and the
 // 11008 x 4096 gate/up pair 48.2 against 37.5 us, hence the line at 2^25 codes (bf16 results only: the
 // warps of the other kernel sum shorter chains, which an f32 result shows).  Of the two warp-MMA
-// kernels the ring kernel (bulk copies into shared memory) wins up to 16 tokens on grids of up to five CTAs per SM
-// (three stages while all CTAs are resident at once, two stages beyond: see launch_ring_one), the register-streaming
-// one on larger grids (32000 x 4096: 37 against 41 us) and above 16 tokens.
+// kernels the ring kernel (bulk copies into shared memory) wins up to 16 tokens, the register-streaming one above.  This rule,
+// and so the planner, names the ring for grids of up to five CTAs per SM only and the family "mma" beyond; the forward
+// then hands up to 16 tokens of that family to the ring as well (ring_kernel_takes_over).
 // f32 activations on SMALL layers (config 1: 784 -> 256 -> 10 at 64 tokens): the whole forward is a few MFLOP and
 // what counts is the number and latency of launches; the CUDA-core GEMV in slices of tokens is one short launch
 // where the tensor-core route never fills (and it keeps every bit of x, which the hi/lo pair does not).

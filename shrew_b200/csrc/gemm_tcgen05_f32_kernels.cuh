@@ -199,6 +199,16 @@ linear_i8_tcgen05_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const f
         const bool relu = (epilogue & 0xFF) == SHREWQ_EPILOGUE_RELU;
         // x may be the previous kernel's output, and y may still be read by it
         pdl_wait();
+        // scale and bias of this lane's channel, requested a tile ahead
+        float sc_next = 0.0f, bs_next = 0.0f;
+        auto channel = [&](int tile) {
+            const int n = (tile % n_tiles) * kF32Chan + quad * 32 + lane;
+            if (tile < end && n < N) {
+                sc_next = __ldg(scales + n);
+                bs_next = bias ? __ldg(bias + n) : 0.0f;
+            }
+        };
+        channel(begin);
         int li = 0, xl0 = 0;
         bool ok = true;
         for (int tile = begin; tile < end && ok; ++tile, ++li) {
@@ -248,56 +258,54 @@ linear_i8_tcgen05_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const f
                 }
                 xl0 += nkb;
             }
-            const bool n_ok = n < N;
-            const float sc = n_ok ? scales[n] : 0.0f, bs = (n_ok && bias) ? bias[n] : 0.0f;
             const int buf = li & 1;
+            const bool n_ok = n < N;
+            const float sc = sc_next, bs = bs_next;
+            channel(tile + 1);
             if (ok) ok = f32_wait_warp(bars + C::kAccFull + 8 * buf, (li >> 1) & 1, ctl, status, 7, buf);
             if (!ok) break;
             tc_fence_after();
-#pragma unroll 1
-            for (int c = 0; c < TOK / 64; ++c) {
-                const int col = half * (TOK / 2) + c * 32;
-                uint32_t r[32];
-                const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + buf * C::kParts * TOK + col;
-                tc_ld32(acc, r);
-                if constexpr (C::kParts == 2) {
-                    if (kb_part < nkb) {
-                        uint32_t r2[32];
-                        tc_ld32(acc + TOK, r2);
-                        tc_wait_ld();
+            // this warp's half of the tokens, all of it into registers, so that the accumulator is free at once
+            constexpr int kChunks = TOK / 64;
+            uint32_t r[kChunks][32];
+            const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + buf * C::kParts * TOK + half * (TOK / 2);
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(r2[i]));
-                    }
-                }
-                tc_wait_ld();
-                if (c == TOK / 64 - 1) {
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bars + C::kAccEmpty + 8 * buf);
-                }
-                if (n_ok) {
-                    float *p = y + (size_t)(m0 + col) * ldy + n;
-                    const int rows = M - (m0 + col) < 32 ? M - (m0 + col) : 32;
-                    if (rows == 32) {
+            for (int c = 0; c < kChunks; ++c) tc_ld32(acc + c * 32, r[c]);
+            if constexpr (C::kParts == 2) {
+                if (kb_part < nkb) {
+                    uint32_t r2[32];
+                    tc_ld32(acc + TOK, r2);
+                    tc_wait_ld();
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            float o = __uint_as_float(r[i]) * sc + bs;
-                            if (relu) o = fmaxf(o, 0.0f);
-                            *p = o;
-                            p += ldy;
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            float o = __uint_as_float(r[i]) * sc + bs;
-                            if (relu) o = fmaxf(o, 0.0f);
-                            if (i < rows) *p = o;
-                            p += ldy;
-                        }
-                    }
+                    for (int i = 0; i < 32; ++i) r[0][i] = __float_as_uint(__uint_as_float(r[0][i]) + __uint_as_float(r2[i]));
                 }
-                __syncwarp();
             }
+            tc_wait_ld();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + C::kAccEmpty + 8 * buf);
+            if (n_ok) {
+                const int m = m0 + half * (TOK / 2), rows = M - m;
+                float *p = y + (size_t)m * ldy + n;
+                if (rows >= TOK / 2) {
+#pragma unroll
+                    for (int i = 0; i < TOK / 2; ++i) {
+                        float o = __uint_as_float(r[i / 32][i % 32]) * sc + bs;
+                        if (relu) o = fmaxf(o, 0.0f);
+                        *p = o;
+                        p += ldy;
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < TOK / 2; ++i) {
+                        float o = __uint_as_float(r[i / 32][i % 32]) * sc + bs;
+                        if (relu) o = fmaxf(o, 0.0f);
+                        if (i < rows) *p = o;
+                        p += ldy;
+                    }
+                }
+            }
+            __syncwarp();
         }
     }
 

@@ -21,8 +21,7 @@
 // A CTA of 8 warps owns 16 channels (8 when gated: a gate block and an up block); the warps
 // split K in 64-wide blocks and their accumulators are summed through shared memory.
 //
-// F16 variant ("mma-f16").  Widening a code to bf16 costs 2.5 instructions (byte-permute into
-// an f32 magic number, subtract, pack two f32 into bf16x2), which at batch 1-4 makes the
+// F16 variant ("mma-f16").  Widening a code to bf16 costs 2.25 instructions (widen_bf16.cuh), which at batch 1-4 makes the
 // kernel issue-bound like the CUDA-core GEMV.  To f16 it costs 1: a byte-permute builds the
 // halves 0x6400 | u (= 1024 + u exactly, u = code + 128), one packed subtract of 1152 leaves
 // the code.  The MMA then needs f16 activations, and f16 has 5 exponent bits where bf16 has

@@ -15,16 +15,16 @@
 //    (full / empty mbarriers).  With S = 8 a whole K = 4096 row block is requested in the kernel's first hundred
 //    cycles; no load instruction waits in a register scoreboard and the bytes in flight per SM (S * 8 KB per
 //    CTA) do not depend on how many warps are resident.
-//  - Four consumer warps split every stage by k (two 64-wide k-blocks each).  The weights are the A operand of
+//  - Eight consumer warps split every stage by k (four 64-wide k-blocks each).  The weights are the A operand of
 //    mma.sync.m16n8k16 (16 rows x 16 k), the activations the B operand (16 k x 8 tokens): widening a code to
-//    bf16 costs 2.5 instructions whatever the batch, and one to four MMAs per step cover 8 to 32 tokens with
+//    bf16 costs 2.25 instructions whatever the batch (widen_bf16.cuh), and one to four MMAs per step cover 8 to 32 tokens with
 //    the same converted fragment.  Lane (g = lane / 4, t = lane % 4) reads the 16 codes [16t, 16t + 16) of
 //    rows g and g + 8 of the k-block and the 16 activations of the same k for tokens g (+ 8, 16, 24); MMA
 //    step j uses codes and activations 4j .. 4j+3 of those runs for A and B alike (a dot product does not care
 //    about the order of k).  Rows are 576 bytes apart in shared memory, so the 16-byte reads of a quarter warp
 //    fall into distinct banks.  Activations come straight from global memory (L1 keeps them: every CTA of
 //    an SM reads the same few KB), requested before the wait for the stage.
-//  - The four warps' accumulators meet in shared memory; 128 (gated: 64) x NT threads apply scale, bias and
+//  - The eight warps' accumulators meet in shared memory; 128 (gated: 64) x NT threads apply scale, bias and
 //    the epilogue and store to the local and the peer destinations.
 //
 // Programmatic dependent launch: the kernel lets its successor start at once, and its producer requests WEIGHTS
