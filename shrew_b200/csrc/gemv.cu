@@ -14,14 +14,6 @@ template <int MT, int R, typename XT, typename YT, bool GATED>
 void launch_one(shrewq_ctx *ctx, const ForwardArgs &a) {
     constexpr int NR = GATED ? R / 2 : R;
     const unsigned gx = (unsigned)((a.N + NR - 1) / NR);
-    if (a.M > (size_t)MT) {
-        // batches above MT tokens run as slices of MT tokens along grid.y (small layers with f32 activations: the
-        // weights come from L2 for every slice but the first)
-        gemv_i8_kernel<MT, R, XT, YT, GATED, false, true><<<dim3(gx, (unsigned)((a.M + MT - 1) / MT)), kThreads, 0, ctx->stream>>>(
-            a.q, a.scales, a.bias, a.q_up, a.scales_up, a.bias_up, static_cast<const XT *>(a.x), static_cast<YT *>(a.y), a.extra,
-            (int)a.M, (int)a.N, (int)a.K, a.ldy, a.epilogue);
-        return;
-    }
     // With a.pdl (and one or two tokens: from four tokens on the early weight fetch costs more registers than the
     // overlap returns) the launch takes the PDL variant of the kernel with programmatic stream serialization:
     // back-to-back GEMVs overlap launch latency, prologue and the first weight loads with the tail of the kernel before.
@@ -53,9 +45,13 @@ void dispatch_m(shrewq_ctx *ctx, const ForwardArgs &a) {
     else if (a.M <= 4) launch_one<4, 4, XT, YT, GATED>(ctx, a);
     else if (a.M <= 8) launch_one<8, 2, XT, YT, GATED>(ctx, a);
     else if (a.M <= 16) launch_one<16, 2, XT, YT, GATED>(ctx, a);
-    // slices: of 4 tokens, since a CTA's own latency is the time of these calls and 16 tokens a thread are 160 shuffles at its
-    // end: 64 x 1024 x 1024 36.1 -> 22.7 us, 40 x 512 x 768 15.4 -> 7.9, 64 x 256 x 784 12 -> 7.5
-    else launch_one<4, 4, XT, YT, GATED>(ctx, a);
+    else {  // slices of tokens along grid.y
+        constexpr int NR = GATED ? 2 : 4;
+        gemv_i8_slices_kernel<XT, YT, GATED><<<dim3((unsigned)((a.N + NR - 1) / NR), (unsigned)((a.M + kSliceTokens - 1) / kSliceTokens)), kThreads,
+                                               0, ctx->stream>>>(
+            a.q, a.scales, a.bias, a.q_up, a.scales_up, a.bias_up, static_cast<const XT *>(a.x), static_cast<YT *>(a.y), a.extra,
+            (int)a.M, (int)a.N, (int)a.K, a.ldy, a.epilogue);
+    }
 }
 
 // ---- the ring kernel (1..32 tokens, bf16 activations): bulk copies into a shared-memory ring + warp MMA ----

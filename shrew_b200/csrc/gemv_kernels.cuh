@@ -25,6 +25,7 @@ namespace {
 
 constexpr int kWarps = 4;
 constexpr int kThreads = kWarps * 32;
+constexpr int kSliceTokens = 4;  // tokens of a slice (gemv_i8_slices_kernel)
 
 // 4 INT8 codes (one word) -> 4 floats, exactly.  Two forms, chosen by the token count of the instantiation:
 //  - integer-to-float conversions: they run on the quarter-rate conversion pipe, which is otherwise idle, so with two
@@ -96,10 +97,7 @@ __device__ __forceinline__ float silu(float g) { return g / (1.0f + __expf(-g));
 // once, fetches its first weights, and only then waits for the previous kernel, whose output its
 // activations may be; the weights never depend on an earlier kernel.  Back-to-back GEMVs thus keep
 // the weight stream going across the kernel boundary.
-// SLICED: the grid's y dimension walks over slices of MT tokens (batches above MT on small layers); a separate
-// instantiation, so that the unsliced kernels keep their code (the slice arithmetic cost them 15-25 % when it was
-// unconditional).
-template <int MT, int R, typename XT, typename YT, bool GATED, bool PDL = false, bool SLICED = false>
+template <int MT, int R, typename XT, typename YT, bool GATED, bool PDL = false>
 __global__ void __launch_bounds__(kThreads)
 gemv_i8_kernel(const int8_t *__restrict__ q, const float *__restrict__ scales,
                const float *__restrict__ bias, const int8_t *__restrict__ q_up,
@@ -108,12 +106,6 @@ gemv_i8_kernel(const int8_t *__restrict__ q, const float *__restrict__ scales,
                size_t ldy, int epilogue) {
     constexpr int NR = GATED ? R / 2 : R;  // distinct output columns per CTA
     if constexpr (PDL) pdl_launch_dependents();
-    int mb = 0;
-    if constexpr (SLICED) {
-        mb = (int)blockIdx.y * MT;
-        x += (size_t)mb * K;
-        M = M - mb < MT ? M - mb : MT;
-    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n0 = blockIdx.x * NR;
     const int chunks = K >> 4;
@@ -214,8 +206,112 @@ gemv_i8_kernel(const int8_t *__restrict__ q, const float *__restrict__ scales,
             out = s * scales[n] + (bias ? bias[n] : 0.0f);
             if (epilogue == SHREWQ_EPILOGUE_RELU) out = fmaxf(out, 0.0f);
         }
-        store_y<YT>(y + (size_t)(mb + m) * ldy + n, out);
-        for (int d = 0; d < extra.n; ++d) store_y<YT>(static_cast<YT *>(extra.p[d]) + (size_t)(mb + m) * ldy + n, out);
+        store_y<YT>(y + (size_t)m * ldy + n, out);
+        for (int d = 0; d < extra.n; ++d) store_y<YT>(static_cast<YT *>(extra.p[d]) + (size_t)m * ldy + n, out);
+    }
+}
+
+// 4 consecutive activations as f32
+template <typename XT>
+__device__ __forceinline__ void load_x4(const XT *p, float *o);
+template <>
+__device__ __forceinline__ void load_x4<float>(const float *p, float *o) {
+    const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
+    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+}
+template <>
+__device__ __forceinline__ void load_x4<__nv_bfloat16>(const __nv_bfloat16 *p, float *o) {
+    const uint2 v = __ldg(reinterpret_cast<const uint2 *>(p));
+    o[0] = __uint_as_float(v.x << 16); o[1] = __uint_as_float(v.x & 0xFFFF0000u);
+    o[2] = __uint_as_float(v.y << 16); o[3] = __uint_as_float(v.y & 0xFFFF0000u);
+}
+
+// More than 16 tokens on small layers: slices of 4 tokens along grid.y, 4 rows (gated: 2 pairs) along grid.x; the weights come
+// from L2 for every slice but the first.  The call is a few MFLOP, so what bounds it is a CTA's own chain of loads, L1 passes and
+// shuffles: a thread takes 4 codes a row and not 16, whose 16 f32 activations 64 bytes apart from lane to lane are sixteen
+// passes of L1 for each load (and at 784 features 79 of 128 threads have no chunk); and the 16 sums of a warp are reduced
+// together, halving what a lane holds at every step, in 16 shuffles instead of 80.  64 x 256 x 784 7.5 -> 5.5 us, 64 x 1024 x 1024
+// 22.7 -> 11.8, 100 x 1000 x 512 28.1 -> 13.7, 64 x 10 x 256 2.6 -> 2.0 (tokens x rows x features; before: 16 codes a thread).
+template <typename XT, typename YT, bool GATED>
+__global__ void __launch_bounds__(kThreads)
+gemv_i8_slices_kernel(const int8_t *__restrict__ q, const float *__restrict__ scales, const float *__restrict__ bias,
+                      const int8_t *__restrict__ q_up, const float *__restrict__ scales_up, const float *__restrict__ bias_up,
+                      const XT *__restrict__ x, YT *__restrict__ y, Dests extra, int M, int N, int K, size_t ldy, int epilogue) {
+    constexpr int MT = kSliceTokens, R = 4, NR = GATED ? R / 2 : R;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n0 = blockIdx.x * NR, mb = blockIdx.y * MT;
+    const int8_t *rowp[R];
+    const XT *xp[MT];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        int n = n0 + (GATED ? (r >> 1) : r);
+        n = n < N ? n : N - 1;  // clamp: duplicates are computed and dropped
+        rowp[r] = ((GATED && (r & 1)) ? q_up : q) + (size_t)n * K;
+    }
+#pragma unroll
+    for (int m = 0; m < MT; ++m) xp[m] = x + (size_t)(mb + m < M ? mb + m : M - 1) * K;
+
+    float v[R * MT];
+#pragma unroll
+    for (int i = 0; i < R * MT; ++i) v[i] = 0.0f;
+#pragma unroll 2
+    for (int k = 4 * threadIdx.x; k < K; k += 4 * kThreads) {
+        uint32_t w[R];
+        float xf[MT][4];
+#pragma unroll
+        for (int r = 0; r < R; ++r) w[r] = __ldg(reinterpret_cast<const uint32_t *>(rowp[r] + k));
+#pragma unroll
+        for (int m = 0; m < MT; ++m) load_x4<XT>(xp[m] + k, xf[m]);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            float wf[4];
+            i8x4_to_f32<true>(w[r], wf);
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[r * MT + m] = fmaf(wf[e], xf[m][e], v[r * MT + m]);
+        }
+    }
+    // a lane hands over the half of its sums that its partner keeps: 8 + 4 + 2 + 1 shuffles, then one for the last pair; it
+    // ends with the sum of index `slot`
+    static_assert(R * MT == 16, "four halvings");
+    __shared__ float s_red[kWarps][16];
+#pragma unroll
+    for (int step = 0; step < 4; ++step) {
+        const int o = 16 >> step, cnt = 8 >> step;
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < cnt; ++i) {
+            const float other = __shfl_xor_sync(0xFFFFFFFFu, up ? v[i] : v[i + cnt], o);
+            v[i] = (up ? v[i + cnt] : v[i]) + other;
+        }
+    }
+    v[0] += __shfl_xor_sync(0xFFFFFFFFu, v[0], 1);
+    const int slot = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+    if ((lane & 1) == 0) s_red[warp][slot] = v[0];
+    __syncthreads();
+
+    if (threadIdx.x < NR * MT) {
+        const int nr = threadIdx.x % NR, m = threadIdx.x / NR, n = n0 + nr;
+        if (n >= N || mb + m >= M) return;
+        auto sum = [&](int r) {
+            float s = 0.0f;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) s += s_red[w][r * MT + m];
+            return s;
+        };
+        float out;
+        if constexpr (GATED) {
+            const float g = sum(2 * nr) * scales[n] + (bias ? bias[n] : 0.0f);
+            const float u = sum(2 * nr + 1) * scales_up[n] + (bias_up ? bias_up[n] : 0.0f);
+            out = silu(g) * u;
+        } else {
+            out = sum(nr) * scales[n] + (bias ? bias[n] : 0.0f);
+            if (epilogue == SHREWQ_EPILOGUE_RELU) out = fmaxf(out, 0.0f);
+        }
+        const size_t off = (size_t)(mb + m) * ldy + n;
+        store_y<YT>(y + off, out);
+        for (int d = 0; d < extra.n; ++d) store_y<YT>(static_cast<YT *>(extra.p[d]) + off, out);
     }
 }
 

@@ -43,6 +43,7 @@
 
 struct emu_uint3 { unsigned x, y, z; };
 struct float4 { float x, y, z, w; };
+struct uint2 { uint32_t x, y; };
 struct uint4 { unsigned x, y, z, w; };
 static inline float4 make_float4(float x, float y, float z, float w) { return float4{x, y, z, w}; }
 static inline uint4 make_uint4(unsigned x, unsigned y, unsigned z, unsigned w) { return uint4{x, y, z, w}; }

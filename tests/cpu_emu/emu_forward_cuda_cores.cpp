@@ -25,15 +25,7 @@ struct Args {
 template <int MT, int R, typename XT, typename YT, bool GATED>
 void gemv_one(const Args &a) {
     constexpr int NR = GATED ? R / 2 : R;
-    const unsigned grid = (unsigned)((a.N + NR - 1) / NR), gy = (unsigned)((a.M + MT - 1) / MT);  // as launch_one
-    if (gy > 1) {  // as launch_one: the sliced instantiation
-        emu::launch3(grid, gy, 1, kThreads, 0, [&] {
-            gemv_i8_kernel<MT, R, XT, YT, GATED, false, true>(a.q, a.scales, a.bias, a.q_up, a.scales_up, a.bias_up,
-                                                              static_cast<const XT *>(a.x), static_cast<YT *>(a.y), g_peers, a.M,
-                                                              a.N, a.K, a.ldy, a.epilogue);
-        });
-        return;
-    }
+    const unsigned grid = (unsigned)((a.N + NR - 1) / NR);  // as launch_one
     // pdl: the variant that fetches its first weights before waiting for the previous kernel
     if (a.pdl)
         emu::launch(grid, kThreads, [&] {
@@ -54,7 +46,11 @@ void gemv_m(const Args &a) {
     else if (a.M <= 4) gemv_one<4, 4, XT, YT, GATED>(a);
     else if (a.M <= 8) gemv_one<8, 2, XT, YT, GATED>(a);
     else if (a.M <= 16) gemv_one<16, 2, XT, YT, GATED>(a);
-    else gemv_one<4, 4, XT, YT, GATED>(a);
+    else
+        emu::launch3((unsigned)((a.N + (GATED ? 1 : 3)) / (GATED ? 2 : 4)), (unsigned)((a.M + kSliceTokens - 1) / kSliceTokens), 1, kThreads, 0, [&] {
+            gemv_i8_slices_kernel<XT, YT, GATED>(a.q, a.scales, a.bias, a.q_up, a.scales_up, a.bias_up, static_cast<const XT *>(a.x),
+                                                 static_cast<YT *>(a.y), g_peers, a.M, a.N, a.K, a.ldy, a.epilogue);
+        });
 }
 template <typename XT, typename YT>
 void gemv_g(const Args &a) {
