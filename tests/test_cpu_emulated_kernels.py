@@ -1057,6 +1057,23 @@ def test_gemv_matches_oracle(oracle, emu_cc, M, x_bf16):
     assert oracle.rel_err(y[:, :N], ref) < 2e-6 and np.all(y[:, N:] == 7.0)
 
 
+# Slices of 4 tokens: the narrowest layers (fewer features than a warp takes, fewer rows than a CTA), features just past one
+# pass of the CTA, a last slice of one token, gate/up pairs.  f32 sums of K products: below K * 2^-24 relative to sum |q||x|.
+@pytest.mark.parametrize("M,N,K,gated,x_bf16", [(17, 1, 16, False, 0), (20, 6, 512, False, 1), (18, 5, 528, True, 0), (128, 3, 48, True, 1),
+                                                (21, 9, 1040, False, 0)])
+def test_gemv_slices_match_oracle(oracle, emu_cc, M, N, K, gated, x_bf16):
+    rng = np.random.default_rng(M + K)
+    mats = [(rng.integers(-128, 128, size=(N, K)).astype(np.int8), rng.random(N) * 1e-2 + 1e-4, (rng.standard_normal(N) * 0.1).astype(np.float32))
+            for _ in range(2)]
+    x32 = rng.standard_normal((M, K)).astype(np.float32)
+    bits, xb = _bf16_bits(x32)
+    x_in, x_ref = (bits, xb) if x_bf16 else (x32, x32)
+    (q, sc, b), up = mats
+    ref = _gated_ref(oracle, q, sc, b, *up, x_ref) if gated else oracle.np_linear_forward(q, sc, oracle.PER_CHANNEL, b, x_ref)
+    y = _cc_forward(emu_cc, 0, q, sc, b, x_in, x_bf16, 0, up=up if gated else None, ldy=N + 2)
+    assert oracle.rel_err(y[:, :N], ref) < 1e-5 and np.all(y[:, N:] == 7.0)
+
+
 @pytest.mark.parametrize("M", [1, 3, 8, 9, 16, 17, 32])
 @pytest.mark.parametrize("y_bf16", [0, 1], ids=["f32-out", "bf16-out"])
 @pytest.mark.parametrize("N,K,kc", [(37, 576, 512), (20, 64 * 137, 512), (20, 64 * 137, 1024), (18, 64 * 137, 2048), (5, 64, 1024)],
