@@ -9,10 +9,10 @@
 namespace shrewq {
 namespace {
 
-template <int TOK>
+template <int TOK, int XKB>
 int launch_f32(shrewq_ctx *ctx, const ForwardArgs &a, const CUtensorMap &tw) {
-    using C = F32Cfg<TOK>;
-    auto kern = linear_i8_tcgen05_f32_kernel<TOK>;
+    using C = F32Cfg<TOK, XKB>;
+    auto kern = linear_i8_tcgen05_f32_kernel<TOK, XKB>;
     static std::atomic<unsigned long long> attr_done{0};  // per instantiation: bit d = device d has the attribute
     const int d = ctx->device;
     if (d < 0 || d >= 64 || !((attr_done.load(std::memory_order_acquire) >> d) & 1ull)) {
@@ -46,9 +46,14 @@ int launch_gemm_tcgen05_f32(shrewq_ctx *ctx, const ForwardArgs &a, const void *w
     const CUtensorMap &tw = *static_cast<const CUtensorMap *>(w_tmap);
     const size_t n_tiles = (a.N + kF32Chan - 1) / kF32Chan, tiles128 = n_tiles * ((a.M + 127) / 128);
     // 128-token tiles as soon as 64-token ones would take two rounds of the SMs: 4096 x 256 x 256 (128 of 64 tokens) 5.6 against
-    // 6.4 us, 4096 x 512 x 512 (256) 13.3 against 9.9 us, 4096 x 50257 x 256 445 against 296 us.  Option tc_tok overrides.
+    // 6.4 us, 4096 x 512 x 512 (256) 13.3 against 9.9 us, 4096 x 50257 x 256 327 against 275 us.  Option tc_tok overrides.
     const bool wide = ctx->tuning.tc_tok == 128 || (ctx->tuning.tc_tok != 64 && 2 * tiles128 > (size_t)ctx->sm_count);
-    return wide ? launch_f32<128>(ctx, a, tw) : launch_f32<64>(ctx, a, tw);
+    // 128 KB for activations (and the rest for a deeper ring of codes) as long as those of a token tile fit there, else 192 KB.
+    // With 128-token tiles only where output rows start on 32-byte sectors: 4096 x 50304 x 256 243 -> 219 us, but at 50257
+    // channels, where every store splits sectors and L2 is the limit, 275 against 292 us.
+    const bool sectors = (a.ldy * sizeof(float)) % 32 == 0 && (reinterpret_cast<uintptr_t>(a.y) & 31) == 0;
+    if (wide) return sectors && a.K <= (size_t)F32Cfg<128, 128>::kXSlots * kF32BlockK ? launch_f32<128, 128>(ctx, a, tw) : launch_f32<128, 192>(ctx, a, tw);
+    return a.K <= (size_t)F32Cfg<64, 128>::kXSlots * kF32BlockK ? launch_f32<64, 128>(ctx, a, tw) : launch_f32<64, 192>(ctx, a, tw);
 }
 
 }  // namespace shrewq

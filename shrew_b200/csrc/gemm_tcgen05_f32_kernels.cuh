@@ -12,7 +12,7 @@
 //  - one CTA per SM walks a contiguous range of output tiles, channel tiles fastest; the accumulators are double
 //    buffered, so the stores of a tile run under the loads, widening and MMAs of the next;
 //  - the activations of a token tile are read as f32, split and swizzled into shared memory by the epilogue warps and
-//    stay there for all channel tiles of the range while K fits (kXSlots blocks of 64: 768 features with 64-token
+//    stay there for all channel tiles of the range while K fits (up to 768 features with 64-token
 //    tiles, 384 with 128); wider layers run them through the same slots as a ring.  No pass over x, no copy of it;
 //  - a warp stores its 32 accumulator lanes as 32 consecutive channels of one token straight from registers: 128-byte
 //    segments whatever the alignment of the output row, no staging tile and no barrier.
@@ -38,14 +38,17 @@ constexpr int kF32Threads = 18 * 32;
 constexpr int kF32Chan = 128;  // output channels per tile = tensor-memory lanes
 constexpr int kF32BlockK = 64;
 
-template <int TOK>
+// XKB: kilobytes of shared memory for activations.  The rest of 224 KB are stages for codes, which come from L2 while the
+// results load it: four stages are one tile of 256 features ahead, twelve are three (gemm_tcgen05_f32.cu has what each gives).
+template <int TOK, int XKB>
 struct F32Cfg {
     static_assert(TOK == 64 || TOK == 128, "two accumulators of TOK columns below the operand columns");
     static constexpr int kXTile = TOK * kF32BlockK * 2;  // one bf16 tile of a 64-wide block
     static constexpr int kXSlot = 2 * kXTile;            // hi, then lo
-    static constexpr int kXSlots = 192 * 1024 / kXSlot;
+    static constexpr int kXSlots = XKB * 1024 / kXSlot;
     static constexpr int kWBytes = kF32Chan * kF32BlockK;
-    static constexpr int kWStages = 4;
+    static constexpr int kWStages = (224 - XKB) * 1024 / kWBytes;
+    static_assert(kWStages % 2 == 0, "a converter group owns every second stage");
     static constexpr int kABase = 256;                   // tensor-memory columns of the widened codes
     static constexpr int kACols = kF32BlockK / 2;
     static constexpr int kAStages = (512 - kABase) / kACols;
@@ -76,12 +79,12 @@ __device__ __forceinline__ bool f32_wait_warp(uint32_t bar, uint32_t parity, Ctl
 
 // resident: the activations of a token tile stay in shared memory for all its channel tiles (K <= kXSlots * 64).
 // x 16-byte aligned, K a multiple of 16; y any f32 rows of stride ldy.
-template <int TOK>
+template <int TOK, int XKB>
 __global__ void __launch_bounds__(kF32Threads, 1)
 linear_i8_tcgen05_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const float *__restrict__ scales,
                              const float *__restrict__ bias, const float *__restrict__ x, float *__restrict__ y, int M, int N,
                              int K, size_t ldy, int epilogue, int n_tiles, int tiles, int resident, DeviceStatus *status) {
-    using C = F32Cfg<TOK>;
+    using C = F32Cfg<TOK, XKB>;
     pdl_launch_dependents();
     SHREWQ_DYNAMIC_SMEM(uint8_t, smem_raw);
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -109,7 +112,7 @@ linear_i8_tcgen05_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const f
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(bars + C::kAccFull + 8 * s, 1);
-            mbar_init(bars + C::kAccEmpty + 8 * s, 8);
+            mbar_init(bars + C::kAccEmpty + 8 * s, 4);
         }
         mbar_fence_init();
     }
@@ -195,20 +198,10 @@ linear_i8_tcgen05_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const f
         }
     } else {
         // ---------------- activations in, results out ----------------
-        const int ew = warp - 10, half = ew >> 2, quad = warp & 3, et = ew * 32 + lane;
+        const int ew = warp - 10, group = ew >> 2, quad = warp & 3, et = ew * 32 + lane;
         const bool relu = (epilogue & 0xFF) == SHREWQ_EPILOGUE_RELU;
         // x may be the previous kernel's output, and y may still be read by it
         pdl_wait();
-        // scale and bias of this lane's channel, requested a tile ahead
-        float sc_next = 0.0f, bs_next = 0.0f;
-        auto channel = [&](int tile) {
-            const int n = (tile % n_tiles) * kF32Chan + quad * 32 + lane;
-            if (tile < end && n < N) {
-                sc_next = __ldg(scales + n);
-                bs_next = bias ? __ldg(bias + n) : 0.0f;
-            }
-        };
-        channel(begin);
         int li = 0, xl0 = 0;
         bool ok = true;
         for (int tile = begin; tile < end && ok; ++tile, ++li) {
@@ -258,54 +251,59 @@ linear_i8_tcgen05_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const f
                 }
                 xl0 += nkb;
             }
-            const int buf = li & 1;
+            // the two groups of four warps take turns by tile (and accumulator), so that the stores of one run under the waits and
+            // the tensor-memory loads of the other (4096 x 50257 x 256: 284 -> 275 us)
+            if ((li & 1) != group) continue;
             const bool n_ok = n < N;
-            const float sc = sc_next, bs = bs_next;
-            channel(tile + 1);
+            const float sc = n_ok ? scales[n] : 0.0f, bs = (n_ok && bias) ? bias[n] : 0.0f;
+            const int buf = li & 1;
             if (ok) ok = f32_wait_warp(bars + C::kAccFull + 8 * buf, (li >> 1) & 1, ctl, status, 7, buf);
             if (!ok) break;
             tc_fence_after();
-            // this warp's half of the tokens, all of it into registers, so that the accumulator is free at once
-            constexpr int kChunks = TOK / 64;
-            uint32_t r[kChunks][32];
-            const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + buf * C::kParts * TOK + half * (TOK / 2);
+#pragma unroll 1
+            for (int c = 0; c < TOK / 32; ++c) {
+                const int col = c * 32;
+                uint32_t r[32];
+                const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + buf * C::kParts * TOK + col;
+                tc_ld32(acc, r);
+                if constexpr (C::kParts == 2) {
+                    if (kb_part < nkb) {
+                        uint32_t r2[32];
+                        tc_ld32(acc + TOK, r2);
+                        tc_wait_ld();
 #pragma unroll
-            for (int c = 0; c < kChunks; ++c) tc_ld32(acc + c * 32, r[c]);
-            if constexpr (C::kParts == 2) {
-                if (kb_part < nkb) {
-                    uint32_t r2[32];
-                    tc_ld32(acc + TOK, r2);
-                    tc_wait_ld();
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) r[0][i] = __float_as_uint(__uint_as_float(r[0][i]) + __uint_as_float(r2[i]));
-                }
-            }
-            tc_wait_ld();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bars + C::kAccEmpty + 8 * buf);
-            if (n_ok) {
-                const int m = m0 + half * (TOK / 2), rows = M - m;
-                float *p = y + (size_t)m * ldy + n;
-                if (rows >= TOK / 2) {
-#pragma unroll
-                    for (int i = 0; i < TOK / 2; ++i) {
-                        float o = __uint_as_float(r[i / 32][i % 32]) * sc + bs;
-                        if (relu) o = fmaxf(o, 0.0f);
-                        *p = o;
-                        p += ldy;
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < TOK / 2; ++i) {
-                        float o = __uint_as_float(r[i / 32][i % 32]) * sc + bs;
-                        if (relu) o = fmaxf(o, 0.0f);
-                        if (i < rows) *p = o;
-                        p += ldy;
+                        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(r2[i]));
                     }
                 }
+                tc_wait_ld();
+                if (c == TOK / 32 - 1) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bars + C::kAccEmpty + 8 * buf);
+                }
+                if (n_ok) {
+                    float *p = y + (size_t)(m0 + col) * ldy + n;
+                    const int rows = M - (m0 + col) < 32 ? M - (m0 + col) : 32;
+                    if (rows == 32) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            float o = __uint_as_float(r[i]) * sc + bs;
+                            if (relu) o = fmaxf(o, 0.0f);
+                            *p = o;
+                            p += ldy;
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            float o = __uint_as_float(r[i]) * sc + bs;
+                            if (relu) o = fmaxf(o, 0.0f);
+                            if (i < rows) *p = o;
+                            p += ldy;
+                        }
+                    }
+                }
+                __syncwarp();
             }
-            __syncwarp();
         }
     }
 

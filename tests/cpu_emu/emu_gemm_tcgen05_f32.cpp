@@ -7,10 +7,10 @@
 
 using namespace shrewq;
 
-template <int TOK>
+template <int TOK, int XKB>
 static int run(const int8_t *q, const float *scales, const float *bias, const float *x, float *y, int M, int N, int K, size_t ldy,
                int epilogue, int ctas) {
-    using C = F32Cfg<TOK>;
+    using C = F32Cfg<TOK, XKB>;
     const CUtensorMap tw{q, 1, (uint64_t)K, (uint64_t)N, (uint64_t)K, (uint32_t)kF32BlockK, 128, 64};
     const int n_tiles = (N + kF32Chan - 1) / kF32Chan, tiles = n_tiles * ((M + TOK - 1) / TOK);
     const int resident = K <= C::kXSlots * kF32BlockK;
@@ -18,7 +18,7 @@ static int run(const int8_t *q, const float *scales, const float *bias, const fl
     DeviceStatus st{0, 0, 0, 0};
     emu::g_failed = false;
     emu::launch3((unsigned)ctas, 1, 1, kF32Threads, C::kSmemBytes, [&] {
-        linear_i8_tcgen05_f32_kernel<TOK>(tw, scales, bias, x, y, M, N, K, ldy, epilogue, n_tiles, tiles, resident, &st);
+        linear_i8_tcgen05_f32_kernel<TOK, XKB>(tw, scales, bias, x, y, M, N, K, ldy, epilogue, n_tiles, tiles, resident, &st);
     });
     if (emu::g_failed) return -4;
     return st.timeout_flag ? -2 : 0;
@@ -27,8 +27,9 @@ static int run(const int8_t *q, const float *scales, const float *bias, const fl
 // x: f32 [M,K]; y: f32 [M, ldy].  Returns 0; -2 when a bounded wait gave up; -4 when a rule of the model was violated.
 extern "C" int emu_gemm_tcgen05_f32(const int8_t *q, const float *scales, const float *bias, const float *x, float *y, int M, int N,
                                     int K, size_t ldy, int epilogue, int tok, int ctas) {
-    return tok == 128 ? run<128>(q, scales, bias, x, y, M, N, K, ldy, epilogue, ctas)
-                      : run<64>(q, scales, bias, x, y, M, N, K, ldy, epilogue, ctas);
+    // shared memory for activations as launch_gemm_tcgen05_f32 chooses it
+    if (tok == 128) return K <= 256 && ldy % 8 == 0 ? run<128, 128>(q, scales, bias, x, y, M, N, K, ldy, epilogue, ctas) : run<128, 192>(q, scales, bias, x, y, M, N, K, ldy, epilogue, ctas);
+    return K <= 512 ? run<64, 128>(q, scales, bias, x, y, M, N, K, ldy, epilogue, ctas) : run<64, 192>(q, scales, bias, x, y, M, N, K, ldy, epilogue, ctas);
 }
 
 extern "C" void emu_drop_tma(int n) {

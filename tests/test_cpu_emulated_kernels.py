@@ -670,7 +670,7 @@ def test_f32_activations_as_hi_lo_pair_on_the_tensor_cores(oracle, emu, emu_tc, 
 # f32, so the relative error stays below 2^-16 + K * 2^-24 of sum |q||x|, with non-negative x below 1e-4 of the result's norm.
 @pytest.mark.parametrize("tok,M,N,K,ldy,ctas,late", [
     (64, 64, 128, 16, 128, 1, 0), (64, 65, 129, 80, 131, 1, 0), (64, 130, 300, 256, 300, 2, 3), (64, 200, 520, 768, 521, 3, 0),
-    (64, 70, 130, 784, 130, 1, 5), (64, 100, 200, 1024, 200, 3, 0), (128, 128, 128, 64, 128, 1, 0), (128, 129, 257, 256, 257, 2, 7),
+    (64, 70, 130, 784, 130, 1, 5), (64, 100, 200, 1024, 200, 3, 0), (128, 128, 128, 64, 128, 1, 0), (128, 129, 257, 256, 257, 2, 7), (128, 140, 300, 256, 304, 1, 3),
     (128, 300, 300, 384, 301, 1, 0), (128, 130, 140, 400, 140, 2, 0)])
 def test_tcgen05_persistent_f32_forward(oracle, tok, M, N, K, ldy, ctas, late):
     L = _build("emu_gemm_tcgen05_f32")
