@@ -1,7 +1,6 @@
 // CPU run of the INT8 symmetric quantize / dequantize kernels (shrew_b200/csrc/quantize_kernels.cuh)
 // under the CUDA stand-in.  TEST INFRASTRUCTURE ONLY; see cuda_shim.h.
 #include "cuda_shim.h"
-struct uint2 { unsigned x, y; };
 #include "../../shrew_b200/csrc/quantize_kernels.cuh"
 #include "../../shrew_b200/csrc/quantize_batch_kernels.cuh"
 
