@@ -41,28 +41,24 @@ namespace shrewq {
 namespace {
 
 constexpr int kLanes = 128;     // TMEM lanes = weight rows per CTA
+constexpr int kTokHalf = 128;   // tokens per CTA (half of the pair's tile)
+constexpr int kTokPair = 256;   // MMA N
 constexpr int kBlockK = 64;     // k per sub-block
 constexpr int kSub = 2;         // sub-blocks per stage (128 k)
 constexpr int kUmmaK = 16;
+constexpr int kStages = 4;
 constexpr int kGroups = 3;      // converter groups of 4 warps
 constexpr int kThreads = 64 + 128 * kGroups;
 constexpr int kWSub = kLanes * kBlockK;          // 8192 B of codes
+constexpr int kXSub = kTokHalf * kBlockK * 2;    // 16384 B of bf16 activations
+constexpr int kStageBytes = kSub * (kWSub + kXSub);  // 49152
 constexpr int kXOff = kSub * kWSub;
 constexpr int kAColsPerStage = kSub * (kBlockK / 2);  // 64
-
-// TOKP: tokens of a pair tile = MMA N
-template <int TOKP>
-struct PairCfg {
-    static constexpr int kTokHalf = TOKP / 2;             // tokens per CTA
-    static constexpr int kXSub = kTokHalf * kBlockK * 2;  // bf16 activations
-    static constexpr int kStageBytes = kSub * (kWSub + kXSub);
-    static constexpr int kStages = TOKP == 256 ? 4 : 6;
-    static constexpr int kABase = TOKP;                   // D occupies the columns below
-    static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 1024;
-    static_assert(kABase + kStages * kAColsPerStage <= 512, "TMEM columns");
-    static_assert(kSmemBytes <= 227 * 1024, "shared memory");
-    static_assert(kStages * kStageBytes >= kGroups * kEpiGroupBytes, "the epilogue's staging tiles reuse the pipeline stages");
-};
+constexpr int kABase = kTokPair;                      // D occupies columns [0,256)
+constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 1024;
+static_assert(kABase + kStages * kAColsPerStage <= 512, "TMEM columns");
+static_assert(kSmemBytes <= 227 * 1024, "shared memory");
+static_assert(kStages * kStageBytes >= kGroups * kEpiGroupBytes, "the epilogue's staging tiles reuse the pipeline stages");
 
 // In-kernel cycle trace (tracing build only): CTA (0,0,0), the pair's leader, stamps clock64() per role
 // and pipeline round; layout and meaning as in the single-CTA kernel.
@@ -89,9 +85,9 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, Ct
 // Split-K (gridDim.z > 1): CTA (x, y, z) walks pipeline rounds [z * rounds_per_split, ...) of its tile
 // and parks its raw accumulators in `partials`; the CTA arriving last at the tile's counter adds the
 // slices in split order, applies the epilogue and resets the counter.  Every CTA of a pair is a tile
-// of its own here (128 lanes x TOKP tokens), so nothing crosses the pair in the reduction.
+// of its own here (128 lanes x 256 tokens), so nothing crosses the pair in the reduction.
 struct SplitK2 {
-    float *partials;         // [tile][split][TOKP tokens][128 lanes] f32
+    float *partials;         // [tile][split][256 tokens][128 lanes] f32
     unsigned int *counters;  // one per CTA tile, zero between launches
     int rounds_per_split;
     // Tile-list mode (pairs_total > 0): the grid is a 1-D list of pair tiles (blockIdx.x / 2) starting at
@@ -104,13 +100,11 @@ struct SplitK2 {
 // GATED: as in the single-CTA kernel, the 128 lanes of a CTA carry 64 rows of a gate matrix (tmap_w,
 // 64-row boxes) and the same 64 rows of an up matrix (tmap_w2); the epilogue pairs lane r with lane
 // r + 64 and writes silu(gate) * up for 64 channels per CTA, 128 per pair.
-template <typename YT, bool GATED, int TOKP = 256>
+template <typename YT, bool GATED>
 __global__ void SHREWQ_CLUSTER_OF_2 __launch_bounds__(kThreads, 1)
 linear_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_w2,
                               const __grid_constant__ CUtensorMap tmap_x, Operands ops, YT *__restrict__ y, Dests extra,
                               int M, int N, int K, size_t ldy, int epilogue, SplitK2 sk, DeviceStatus *status) {
-    using C = PairCfg<TOKP>;
-    constexpr int kStages = C::kStages, kStageBytes = C::kStageBytes, kXSub = C::kXSub, kABase = C::kABase;
     constexpr int kChan = GATED ? kLanes / 2 : kLanes;  // output channels per CTA
     TRACE2_INIT
     pdl_launch_dependents();  // the next kernel of the stream may start its prologue (a no-op in an ordinary launch)
@@ -135,8 +129,8 @@ linear_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const 
         pair = t / (int)gridDim.y;
     }
     const int n0 = pair * 2 * kChan + (int)rank * kChan;      // this CTA's first channel
-    const int m0 = m_tile * TOKP + (int)rank * C::kTokHalf;  // this CTA's first token (B half)
-    const int m0_pair = m_tile * TOKP;
+    const int m0 = m_tile * kTokPair + (int)rank * kTokHalf;  // this CTA's first token (B half)
+    const int m0_pair = m_tile * kTokPair;
     const int rounds_total = (K + kBlockK * kSub - 1) / (kBlockK * kSub);
     const int r_begin = (int)blockIdx.z * sk.rounds_per_split;
     const int rounds = min(rounds_total - r_begin, sk.rounds_per_split);  // >= 1 by construction of the grid
@@ -225,8 +219,8 @@ linear_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const 
     } else if (warp == 1) {
         // ---------------- MMA issuer (one thread of the leader CTA) ----------------
         if (rank == 0 && elect_one()) {
-            // D=f32, A=bf16 (K-major, TMEM), B=bf16 (K-major), M=256 (two CTAs), N=TOKP
-            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TOKP >> 3) << 17) |
+            // D=f32, A=bf16 (K-major, TMEM), B=bf16 (K-major), M=256 (two CTAs), N=256
+            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTokPair >> 3) << 17) |
                                        ((uint32_t)((2 * kLanes) >> 4) << 24);
             const uint64_t bdesc0 = make_b_desc(smem_base + kXOff);
             const uint32_t a0 = tmem_base + kABase;
@@ -292,16 +286,16 @@ linear_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const 
             if (lane == 0) mbar_arrive_cluster(aready_leader + s * 8);
             if (quad == 0) TRACE2(2, i, 3);
         }
-        // epilogue: this CTA's channels x the pair's TOKP tokens; 16-column chunks dealt to the groups
+        // epilogue: this CTA's channels x the pair's 256 tokens; 16-column chunks dealt to the groups
         pdl_wait();  // outputs, partial sums and counters may still be in use by the previous kernel of the stream
         if (ok) ok = mbar_wait_warp(bars_u32 + kAcc, 0, ctl, status, 4, 0);
         if (ok) tc_fence_after();
         const int splits = (int)gridDim.z;
         if (splits > 1) {
             const size_t tile = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
-            float *mine = sk.partials + (tile * splits + blockIdx.z) * (size_t)(TOKP * kLanes);
+            float *mine = sk.partials + (tile * splits + blockIdx.z) * (size_t)(kTokPair * kLanes);
             if (ok) {
-                dump_partials<TOKP, kGroups>(tmem_base, mine, group, quad, lane);
+                dump_partials<kTokPair, kGroups>(tmem_base, mine, group, quad, lane);
             }
             __threadfence();
             named_bar_sync(1, 128 * kGroups);
@@ -312,14 +306,14 @@ linear_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const 
             named_bar_sync(1, 128 * kGroups);
             if (*s_is_last) {
                 __threadfence();
-                epilogue_tile<TOKP, kGroups, GATED, YT>(tmem_base, smem, group, quad, lane, ok, ops, y, extra, M, N, ldy, epilogue,
+                epilogue_tile<kTokPair, kGroups, GATED, YT>(tmem_base, smem, group, quad, lane, ok, ops, y, extra, M, N, ldy, epilogue,
                                                             n0, m0_pair,
-                                                            PartialSums{sk.partials + tile * splits * (size_t)(TOKP * kLanes), splits, (size_t)(TOKP * kLanes)});
+                                                            PartialSums{sk.partials + tile * splits * (size_t)(kTokPair * kLanes), splits, (size_t)(kTokPair * kLanes)});
                 named_bar_sync(1, 128 * kGroups);
                 if (threadIdx.x == 64) sk.counters[tile] = 0;  // ready for the next launch
             }
         } else {
-            epilogue_tile<TOKP, kGroups, GATED, YT>(tmem_base, smem, group, quad, lane, ok, ops, y, extra, M, N, ldy, epilogue, n0,
+            epilogue_tile<kTokPair, kGroups, GATED, YT>(tmem_base, smem, group, quad, lane, ok, ops, y, extra, M, N, ldy, epilogue, n0,
                                                         m0_pair, PartialSums{nullptr, 0, 0});
         }
     }

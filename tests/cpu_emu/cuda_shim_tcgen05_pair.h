@@ -42,20 +42,20 @@ static inline void tc_mma_ts_pair_now(uint32_t d_tmem, uint32_t a_tmem, uint64_t
     emu::Block *me = emu::g_block;
     EMU_CHECK(me->rank == 0, "the leader CTA issues the pair MMA");
     const uint32_t N = ((idesc >> 17) & 0x3Fu) << 3, Mrows = ((idesc >> 24) & 0x1Fu) << 4;
-    EMU_CHECK(Mrows == 256 && (N == 128 || N == 256), "Mrows == 256 && (N == 128 || N == 256)");
+    EMU_CHECK(Mrows == 256 && N == 256, "Mrows == 256 && N == 256");
     const uint32_t a_fmt = (idesc >> 7) & 7u;  // 0 = f16, 1 = bf16
     emu::g_last_a_format = (int)a_fmt;
     EMU_CHECK(((idesc >> 4) & 3u) == 1 && a_fmt <= 1 && ((idesc >> 10) & 7u) == 1, "D f32, A f16 or bf16, B bf16");
     EMU_CHECK(((b_desc >> 61) & 7u) == 2 && ((b_desc >> 46) & 1u) == 1, "128-byte swizzle, descriptor version 1");
     const uint32_t start = (uint32_t)(b_desc & 0x3FFFu) << 4, sbo = (uint32_t)((b_desc >> 32) & 0x3FFFu) << 4;
     const uint32_t dcol = d_tmem & 0xFFFF, acol = a_tmem & 0xFFFF;
-    if (!((d_tmem >> 16) == 0 && (a_tmem >> 16) == 0 && dcol + N <= 512 && acol + 8 <= 512 && (N == 128 || N == 256) && Mrows == 256)) {
-        emu::fail("pair tcgen05.mma operands outside tensor memory or not 256 x 128 or 256");
+    if (!((d_tmem >> 16) == 0 && (a_tmem >> 16) == 0 && dcol + N <= 512 && acol + 8 <= 512 && N == 256 && Mrows == 256)) {
+        emu::fail("pair tcgen05.mma operands outside tensor memory or not 256 x 256");
         return;
     }
     std::vector<float> b((size_t)N * 16);
     for (uint32_t n = 0; n < N; ++n) {
-        const uint32_t owner = n / (N / 2), row = n % (N / 2);  // each CTA holds half of B's rows
+        const uint32_t owner = n >> 7, row = n & 127;
         const uint32_t base = smem_u32(me->cluster[owner]->dyn);
         for (uint32_t k = 0; k < 16; ++k) {
             const uint32_t addr = (base | start) + (row >> 3) * sbo + (row & 7) * 128 + k * 2;

@@ -9,27 +9,27 @@
 using namespace shrewq;
 
 namespace {
-template <typename YT, bool GATED, int TOKP>
-int run_tok(const int8_t *q, const int8_t *q_up, const Operands &ops, const uint16_t *x, void *y, int M, int N, int K, size_t ldy,
+template <typename YT, bool GATED>
+int run(const int8_t *q, const int8_t *q_up, const Operands &ops, const uint16_t *x, void *y, int M, int N, int K, size_t ldy,
         int epilogue, int splits, int tile_list, DeviceStatus *st) {
     const uint32_t box_rows = GATED ? 64 : 128;
     const CUtensorMap tw{q, 1, (uint64_t)K, (uint64_t)N, (uint64_t)K, kBlockK, box_rows, 64};
     const CUtensorMap tw2{GATED ? q_up : q, 1, (uint64_t)K, (uint64_t)N, (uint64_t)K, kBlockK, box_rows, 64};
-    const CUtensorMap tx{x, 2, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, kBlockK, PairCfg<TOKP>::kTokHalf, 128};
+    const CUtensorMap tx{x, 2, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, kBlockK, kTokHalf, 128};
     const int chan_pair = GATED ? kLanes : 2 * kLanes;
     const unsigned pairs = (unsigned)((N + chan_pair - 1) / chan_pair);
     Dests none{};
-    const unsigned m_tiles = (unsigned)((M + TOKP - 1) / TOKP);
+    const unsigned m_tiles = (unsigned)((M + kTokPair - 1) / kTokPair);
     const int rounds = (K + kBlockK * kSub - 1) / (kBlockK * kSub);
     if (splits < 1) splits = 1;
     const int rps = (rounds + splits - 1) / splits;
     splits = (rounds + rps - 1) / rps;  // no empty split
     const size_t ctas = (size_t)2 * pairs * m_tiles;
-    std::vector<float> partials(splits > 1 ? ctas * splits * TOKP * kLanes : 0, -12345.0f);
+    std::vector<float> partials(splits > 1 ? ctas * splits * kTokPair * kLanes : 0, -12345.0f);
     std::vector<unsigned int> counters(ctas, 0u);
     SplitK2 sk{splits > 1 ? partials.data() : nullptr, splits > 1 ? counters.data() : nullptr, rps, 0, 0};
     auto body = [&] {
-        linear_i8_tcgen05_pair_kernel<YT, GATED, TOKP>(tw, tw2, tx, ops, static_cast<YT *>(y), none, M, N, K, ldy, epilogue, sk, st);
+        linear_i8_tcgen05_pair_kernel<YT, GATED>(tw, tw2, tx, ops, static_cast<YT *>(y), none, M, N, K, ldy, epilogue, sk, st);
     };
     if (tile_list >= 2) {
         // the two-launch scheme of launch_pair for a short last wave, `tile_list` standing for the pair tiles
@@ -37,28 +37,20 @@ int run_tok(const int8_t *q, const int8_t *q_up, const Operands &ops, const uint
         const int tiles = (int)(pairs * m_tiles), rem = tiles % tile_list;
         if (tiles <= tile_list || rem == 0) return -1;
         sk = SplitK2{nullptr, nullptr, rounds, 0, (int)pairs};
-        emu::launch_cluster2(2u * (unsigned)(tiles - rem), 1, 1, kThreads, PairCfg<TOKP>::kSmemBytes, body);
+        emu::launch_cluster2(2u * (unsigned)(tiles - rem), 1, 1, kThreads, kSmemBytes, body);
         sk = SplitK2{splits > 1 ? partials.data() : nullptr, splits > 1 ? counters.data() : nullptr, rps, tiles - rem, (int)pairs};
-        emu::launch_cluster2(2u * (unsigned)rem, 1, (unsigned)splits, kThreads, PairCfg<TOKP>::kSmemBytes, body);
+        emu::launch_cluster2(2u * (unsigned)rem, 1, (unsigned)splits, kThreads, kSmemBytes, body);
     } else if (tile_list == 1) {  // the 1-D tile list as one launch over all pair tiles
         sk.pairs_total = (int)pairs;
-        emu::launch_cluster2(2 * pairs * m_tiles, 1, (unsigned)splits, kThreads, PairCfg<TOKP>::kSmemBytes, body);
+        emu::launch_cluster2(2 * pairs * m_tiles, 1, (unsigned)splits, kThreads, kSmemBytes, body);
     } else {
-        emu::launch_cluster2(2 * pairs, m_tiles, (unsigned)splits, kThreads, PairCfg<TOKP>::kSmemBytes, body);
+        emu::launch_cluster2(2 * pairs, m_tiles, (unsigned)splits, kThreads, kSmemBytes, body);
     }
     for (unsigned int c : counters)
         if (c != 0) return -3;  // the kernel leaves the tile counters at zero for the next launch
     return 0;
 }
-int g_tok = 256;  // tokens of a pair tile
-template <typename YT, bool GATED, typename... A>
-int run(A... a) {
-    return g_tok == 128 ? run_tok<YT, GATED, 128>(a...) : run_tok<YT, GATED, 256>(a...);
-}
 }  // namespace
-
-// 128- or 256-token pair tiles for the next launches (128 with tile_list >= 2: the last wave as halves)
-extern "C" void emu_pair_tok(int tok) { g_tok = tok; }
 
 extern "C" int emu_last_a_format() { return emu::g_last_a_format.load(); }  // 0 = f16, 1 = bf16
 

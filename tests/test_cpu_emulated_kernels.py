@@ -886,36 +886,6 @@ def test_cta_pair_wait_that_runs_out_ends_both_blocks():
         assert rc == -2, drop
 
 
-# The CTA-pair kernel on 128-token tiles: one and several, ragged tokens and channels, split along K, two-launch tail.
-# bf16 products are exact in the f32 accumulator: the bound is that of its rounding, K * 2^-24 relative to sum |q||x|.
-@pytest.mark.parametrize("M,N,K,gated,splits,tile_list", [
-    (128, 256, 128, False, 1, 0), (130, 300, 784, False, 1, 0), (260, 256, 2048, False, 2, 0), (90, 140, 256, True, 1, 0),
-    (300, 520, 256, False, 2, 4), (257, 260, 144, True, 1, 0)])
-def test_tcgen05_pair_half_tiles(oracle, emu_pair, M, N, K, gated, splits, tile_list):
-    rng = np.random.default_rng(M + N + K)
-    xb, x32 = _bf16_bits(rng.standard_normal((M, K)).astype(np.float32))
-    xa = _aligned((M, K), np.uint16)
-    xa[...] = xb
-    mats = []
-    for _ in range(2 if gated else 1):
-        q = _aligned((N, K), np.int8)
-        q[...] = rng.integers(-128, 128, size=(N, K)).astype(np.int8)
-        mats.append((q, (rng.random(N) * 1e-2 + 1e-4), (rng.standard_normal(N) * 0.1).astype(np.float32)))
-    s32 = [m[1].astype(np.float32) for m in mats]
-    up = (_p(mats[1][0]), _p(s32[1]), _p(mats[1][2])) if gated else (None, None, None)
-    y = np.full((M, N), 7.0, np.float32)
-    emu_pair.emu_pair_tok.argtypes = [_ci]
-    emu_pair.emu_pair_tok(128)
-    try:
-        rc = emu_pair.emu_gemm_tcgen05_pair(_p(mats[0][0]), _p(s32[0]), _p(mats[0][2]), *up, _p(xa), _p(y), M, N, K, N, 0, 0, splits, tile_list)
-    finally:
-        emu_pair.emu_pair_tok(256)
-    assert rc == 0
-    ref = [oracle.np_linear_forward(q, s, oracle.PER_CHANNEL, b, x32) for q, s, b in mats]
-    ref = ref[0] / (1 + np.exp(-ref[0].astype(np.float64))) * ref[1] if gated else ref[0]
-    assert oracle.rel_err(y, ref) < 2e-5
-
-
 def test_tcgen05_two_launch_tail_split(oracle, emu_tc):
     # the tail split (option tc_tailsplit): with "5 SMs", 12 tiles = two full waves as whole-K tiles
     # plus 2 tiles split along K in a second launch; both launches index tiles through the 1-D list
