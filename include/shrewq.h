@@ -99,7 +99,7 @@ SHREWQ_API int shrewq_ctx_set_stream(shrewq_ctx *ctx, void *stream);
  *   "tc_f32"       0..2   the persistent kernel for f32 activations and outputs: 0 never, 1 where it wins by
  *                         measurement (default), 2 whenever it can take the call
  *   "ring_stages"  0, 2, 3  stages of the ring kernel's shared-memory ring (default 0 = three while all its CTAs are
- *                         resident at once, two for larger grids)
+ *                         resident at once, two for larger grids; above 16 tokens the number is fixed)
  *   "pdl"          0/1    programmatic dependent launch of the forward kernels (default 1): from a handle's second
  *                         forward on, a forward kernel may start while the previous kernel of the stream still runs
  *                         and request its WEIGHTS; it reads activations and writes outputs, partial sums and
@@ -366,8 +366,7 @@ SHREWQ_API int shrewq_force_kernel(const char *name);
 /* Which kernel family and launch plan a forward of this shape would get on a GPU with `sm_count` SMs
  * (16-byte aligned buffers, no forced kernel): writes the family name into `kernel` (at least 16 bytes)
  * and, for "tcgen05", the token tile, the tile grid, the K splits and the pipeline rounds per split
- * (zeros otherwise).  "mma" stands for both warp-MMA kernels: up to 16 tokens its calls run on the ring kernel, and two
- * tokens of "gemv" do on large weights with bf16 results.  Pure host arithmetic: needs no GPU and no context.  For tests, benchmarks and
+ * (zeros otherwise).  Pure host arithmetic: needs no GPU and no context.  For tests, benchmarks and
  * capacity planning; no counterpart in the reference. */
 SHREWQ_API int shrewq_plan_forward(size_t M, size_t N, size_t K, int x_is_bf16, int gated, int sm_count, char *kernel,
                         size_t kernel_len, int *tok, int *n_tiles, int *m_tiles, int *splits,

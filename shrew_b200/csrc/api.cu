@@ -201,14 +201,12 @@ const char *shrewq_last_error(const shrewq_ctx *ctx) { return ctx ? ctx->err : g
 uint64_t shrewq_ctx_launch_count(const shrewq_ctx *ctx) { return ctx ? ctx->launches.load() : 0; }
 
 // The default kernel family of a forward with bf16 activations: the one rule, shared by forward_impl and
-// shrewq_plan_forward.  Measured on 4096 x 4096, 11008 x 4096, 4096 x 11008, 1376 x 4096 and 32000 x 4096: the
-// CUDA-core GEMV wins up to 2 tokens, a warp-MMA kernel from 3 to 16 and on small weights to 32, the tcgen05 kernel above:
-// at 24 tokens 4096 x 4096 takes 11.4 us on warp MMA and 11.1 on tcgen05, but 4096 x 11008 25.5 against 17.1 us and the
-// 11008 x 4096 gate/up pair 48.2 against 37.5 us, hence the line at 2^25 codes (bf16 results only: the
-// warps of the other kernel sum shorter chains, which an f32 result shows).  Of the two warp-MMA
-// kernels the ring kernel (bulk copies into shared memory) wins up to 16 tokens, the register-streaming one above.  This rule,
-// and so the planner, names the ring for grids of up to five CTAs per SM only and the family "mma" beyond; the forward
-// then hands up to 16 tokens of that family to the ring as well (ring_kernel_takes_over).
+// shrewq_plan_forward; the type of the result has no part in it.  Measured on 4096 x 4096, 11008 x 4096, 4096 x 11008, 1376 x 4096
+// and 32000 x 4096: the CUDA-core GEMV wins up to 2 tokens, the ring kernel (warp MMA on weights that bulk copies bring into
+// shared memory) from 3 to 32, the tcgen05 kernel above.  The ring against warp MMA with the weights streamed through registers
+// (family "mma", by name only): at 8 tokens 4096 x 4096 6.1 against 13.0 us, gate/up 11008 x 4096 21 against 40, at 24 tokens
+// 8.1 against 11.3 and 31 against 48, with the same sums.  (tcgen05 takes 31 us there too, but in one chain per split, not eight
+// per row: its f32 results are off by 1.0e-6 against 1.2e-7, and its splits need the context's workspace.)
 // f32 activations on SMALL layers (config 1: 784 -> 256 -> 10 at 64 tokens): the whole forward is a few MFLOP and
 // what counts is the number and latency of launches; the CUDA-core GEMV in slices of tokens is one short launch
 // where the tensor-core route never fills (and it keeps every bit of x, which the hi/lo pair does not).
@@ -216,21 +214,14 @@ constexpr size_t kGemvSlicedMaxTokens = 128;
 static bool gemv_slices_win(size_t M, size_t N, size_t K) {
     return M > 16 && M <= kGemvSlicedMaxTokens && M * N * K <= ((size_t)1 << 26);
 }
-static bool ring_kernel_wins(size_t M, size_t N, bool gated, int sm_count) {
-    const size_t ctas = (N + (gated ? 7 : 15)) / (gated ? 8 : 16);
-    return M >= 3 && M <= 16 && ctas <= (size_t)5 * sm_count;
+// Two tokens on large weights with bf16 results: the ring kernel (25.6 -> 20.4 us on the gate/up pair 11008 x 4096).
+static bool two_tokens_on_ring(size_t M, size_t N, size_t K, bool gated, bool y_bf16) {
+    return M == 2 && y_bf16 && N * K * (gated ? 2 : 1) >= ((size_t)1 << 25);
 }
-// Calls of the other small-batch families that the ring kernel runs faster since a CTA walks several row blocks: up to 16
-// tokens every warp-MMA call (gate/up 11008 x 4096 at 8 tokens 40.3 -> 21.3 us, 32000 x 4096 50.1 -> 30.6), and two tokens on
-// weights from 2^25 codes with bf16 results (25.6 -> 20.4 and 35.2 -> 28.0 us; at one token the GEMV stays ahead: 19.4 against 20.2 us).
-static bool ring_kernel_takes_over(int family, size_t M, size_t N, size_t K, bool gated, bool y_bf16) {
-    return (family == kForceMma && M <= 16) || (family == kForceGemv && M == 2 && y_bf16 && N * K * (gated ? 2 : 1) >= ((size_t)1 << 25));
-}
-static int default_family(size_t M, size_t N, size_t K, bool gated, bool y_bf16, int sm_count, bool gemv_ok, bool mma_ok,
-                          bool tc_ok) {
+static int default_family(size_t M, size_t N, size_t K, bool gated, bool y_bf16, bool gemv_ok, bool mma_ok, bool tc_ok) {
+    if (mma_ok && two_tokens_on_ring(M, N, K, gated, y_bf16)) return kForceRing;
     if (gemv_ok && (M <= 2 || (!mma_ok && (M <= 4 || !tc_ok)))) return kForceGemv;
-    if (mma_ok && tc_ok && y_bf16 && M > 16 && M <= 32 && N * K * (gated ? 2 : 1) >= ((size_t)1 << 25)) return kForceTc;
-    if (mma_ok && M <= 32) return ring_kernel_wins(M, N, gated, sm_count) ? kForceRing : kForceMma;
+    if (mma_ok && M <= 32) return kForceRing;
     return tc_ok ? kForceTc : (gemv_ok ? kForceGemv : kForceSimt);
 }
 
@@ -256,7 +247,7 @@ int shrewq_plan_forward(size_t M, size_t N, size_t K, int x_is_bf16, int gated, 
     const bool small = M < (1u << 31) && N < (1u << 31) && K < (1u << 31);
     const bool tc_ok = x_is_bf16 && vec16 && M >= 1 && small;
     const bool mma_ok = x_is_bf16 && (K % 64) == 0 && M <= 64 && small;
-    int fam = default_family(M, N, K, gated != 0, true, sm_count, vec16 && M <= 16, mma_ok, tc_ok);
+    int fam = default_family(M, N, K, gated != 0, false, vec16 && M <= 16, mma_ok, tc_ok);
     if (!x_is_bf16 && vec16 && small && M > 16 && !gated) fam = kForceTcF32;   // f32 activations: the hi/lo tensor-core pass
     if (!x_is_bf16 && vec16 && small && gemv_slices_win(M, N, K)) fam = kForceGemv;
     if (fam == kForceTc && M > 128 && pair_kernel_wins(M, N, K, gated != 0)) fam = kForceTc2Cta;
@@ -696,8 +687,7 @@ static int forward_impl(shrewq_linear *lin, shrewq_linear *up, const void *x_dev
             } else if (M > 128 && tc_ok && (ctx->tuning.tc_pair == 2 || (ctx->tuning.tc_pair == 1 && pair_kernel_wins(M, lin->n, lin->k, up != nullptr)))) {
                 choice = kForceTc2Cta;
             } else {
-                choice = default_family(M, lin->n, lin->k, up != nullptr, a.y_dtype == SHREWQ_BF16, ctx->sm_count, gemv_ok, mma_ok, tc_ok);
-                if (ring_kernel_takes_over(choice, M, lin->n, lin->k, up != nullptr, a.y_dtype == SHREWQ_BF16) && gemv_ring_supported(a)) choice = kForceRing;
+                choice = default_family(M, lin->n, lin->k, up != nullptr, a.y_dtype == SHREWQ_BF16, gemv_ok, mma_ok, tc_ok);
             }
     }
     const char *name;

@@ -110,17 +110,17 @@ int launch_cfg(shrewq_ctx *ctx, const ForwardArgs &a, const CUtensorMap &tw, con
     const LaunchPlan p = plan_launch<TOK, KSUB>(a, GATED ? 64 : 128, ctx->sm_count, allow_split, fixed_scratch ? 64 : 256);
     SplitK sk{nullptr, nullptr, p.rounds_per_split, 0, 0};
     Operands ops{a.scales, a.bias, a.scales_up, a.bias_up};
-    // A short last wave of tiles goes out as a second launch split along K, so that it also fills the SMs: by default for
-    // token tiles up to 64, whose partial sums are small (11008 gate/up channels at 24 tokens are 172 tiles on 148 SMs:
-    // 37.6 -> 31.5 us), with option tc_tailsplit = 1 for all tiles.
-    constexpr bool kSmallTile = TOK <= 64;
-    const bool tail_split = ctx->tuning.tc_tailsplit == 1 || (ctx->tuning.tc_tailsplit == 0 && kSmallTile);
-    if (tail_split && !fixed_scratch && p.splits == 1) {
+    // Option tc_tailsplit: when large tiles leave a short last wave, issue the full waves as one
+    // launch and the tiles of the last wave as a second launch split along K so that it also fills
+    // the SMs.  Not by default: it would make shapes that need no workspace share the context's (between streams,
+    // under capture).
+    const bool tail_split = ctx->tuning.tc_tailsplit == 1;
+    if (tail_split && !fixed_scratch && TOK >= 128 && p.splits == 1) {
         const int tiles = p.n_tiles * p.m_tiles, rem = tiles % ctx->sm_count;
         const int rounds = p.rounds_per_split;
         int s_tail = rem > 0 ? ctx->sm_count / rem : 0;
-        if (s_tail > (kSmallTile ? 8 : 4)) s_tail = kSmallTile ? 8 : 4;
-        if (s_tail > rounds / (kSmallTile ? 4 : 8)) s_tail = rounds / (kSmallTile ? 4 : 8);
+        if (s_tail > 4) s_tail = 4;
+        if (s_tail > rounds / 8) s_tail = rounds / 8;
         if (tiles > ctx->sm_count && rem > 0 && s_tail >= 2) {
             const size_t part_bytes = (size_t)rem * s_tail * TOK * kTileN * sizeof(float);
             if ((rc = ensure_scratch(ctx, kScratchPartialOff + part_bytes)) != SHREWQ_OK) return rc;

@@ -55,11 +55,11 @@ void dispatch_m(shrewq_ctx *ctx, const ForwardArgs &a) {
 }
 
 // ---- the ring kernel (1..32 tokens, bf16 activations): bulk copies into a shared-memory ring + warp MMA ----
-template <int NT, typename YT, bool GATED, int STAGES>
+template <int NT, typename YT, bool GATED, int STAGES, int CHAINS>
 int launch_ring_stages(shrewq_ctx *ctx, const ForwardArgs &a) {
     constexpr int NCH = GATED ? kRingRows / 2 : kRingRows;
     constexpr size_t kSmem = RingCfg<kRingKC, STAGES>::kSmemBytes;
-    auto kern = gemv_i8_ring_kernel<NT, kRingKC, kRingConsumers, YT, GATED, STAGES>;
+    auto kern = gemv_i8_ring_kernel<NT, kRingKC, kRingConsumers, YT, GATED, STAGES, CHAINS>;
     static std::atomic<unsigned long long> attr_done{0};  // per instantiation: bit d = device d has the attribute
     const int d = ctx->device;
     if (d < 0 || d >= 64 || !((attr_done.load(std::memory_order_acquire) >> d) & 1ull)) {
@@ -67,7 +67,7 @@ int launch_ring_stages(shrewq_ctx *ctx, const ForwardArgs &a) {
         if (d >= 0 && d < 64) attr_done.fetch_or(1ull << d, std::memory_order_release);
     }
     cudaLaunchConfig_t cfg = {};
-    const size_t blocks = (a.N + NCH - 1) / NCH, resident = (size_t)(STAGES == 2 ? 3 : 2) * ctx->sm_count;
+    const size_t blocks = (a.N + NCH - 1) / NCH, resident = (size_t)(NT <= 2 && STAGES == 2 ? 3 : 2) * ctx->sm_count;
     cfg.gridDim = dim3((unsigned)(blocks < resident ? blocks : resident));
     cfg.blockDim = dim3((kRingConsumers + 1) * 32);
     cfg.dynamicSmemBytes = kSmem;
@@ -83,22 +83,31 @@ int launch_ring_stages(shrewq_ctx *ctx, const ForwardArgs &a) {
     return SHREWQ_OK;
 }
 
-// three stages (two CTAs per SM) while all CTAs are resident at once, two stages (three CTAs per SM) for larger grids
-template <int NT, typename YT, bool GATED>
+// Up to 16 tokens three stages (two CTAs per SM) while all CTAs are resident at once, two stages (three CTAs per SM) for larger
+// grids.  Above, the registers allow two CTAs per SM: three stages, and two where the reduction buffer of 32 tokens would push
+// the second CTA out (25 to 32 tokens on the gate/up pair 11008 x 4096: 55 us with one CTA per SM).
+template <int NT, int CHAINS, typename YT, bool GATED>
 int launch_ring_one(shrewq_ctx *ctx, const ForwardArgs &a) {
-    constexpr int NCH = GATED ? kRingRows / 2 : kRingRows;
-    const size_t ctas = (a.N + NCH - 1) / NCH;
-    const int stages = ctx->tuning.ring_stages == 2 || ctx->tuning.ring_stages == 3 ? ctx->tuning.ring_stages
-                                                                                     : (ctas <= (size_t)2 * ctx->sm_count ? 3 : 2);
-    if (stages == 2) return launch_ring_stages<NT, YT, GATED, 2>(ctx, a);
-    return launch_ring_stages<NT, YT, GATED, 3>(ctx, a);
+    if constexpr (NT >= 3) {
+        return launch_ring_stages<NT, YT, GATED, NT == 3 ? 3 : 2, CHAINS>(ctx, a);
+    } else {
+        constexpr int NCH = GATED ? kRingRows / 2 : kRingRows;
+        const size_t ctas = (a.N + NCH - 1) / NCH;
+        const int stages = ctx->tuning.ring_stages == 2 || ctx->tuning.ring_stages == 3 ? ctx->tuning.ring_stages
+                                                                                         : (ctas <= (size_t)2 * ctx->sm_count ? 3 : 2);
+        if (stages == 2) return launch_ring_stages<NT, YT, GATED, 2, CHAINS>(ctx, a);
+        return launch_ring_stages<NT, YT, GATED, 3, CHAINS>(ctx, a);
+    }
 }
 
+// Chains of a warp's sums: two up to 16 tokens; one above, which are the sums (bit for bit) of the register-streaming kernel
+// that ran these calls before.
 template <typename YT, bool GATED>
 int launch_ring_m(shrewq_ctx *ctx, const ForwardArgs &a) {
-    if (a.M <= 8) return launch_ring_one<1, YT, GATED>(ctx, a);
-    if (a.M <= 16) return launch_ring_one<2, YT, GATED>(ctx, a);
-    return launch_ring_one<4, YT, GATED>(ctx, a);
+    if (a.M <= 8) return launch_ring_one<1, 2, YT, GATED>(ctx, a);
+    if (a.M <= 16) return launch_ring_one<2, 2, YT, GATED>(ctx, a);
+    if (a.M <= 24) return launch_ring_one<3, 1, YT, GATED>(ctx, a);
+    return launch_ring_one<4, 1, YT, GATED>(ctx, a);
 }
 
 }  // namespace

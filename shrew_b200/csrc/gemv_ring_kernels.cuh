@@ -91,9 +91,12 @@ __device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity, DeviceS
 }
 
 // NT: token blocks of 8 (M <= 8 * NT).  K a multiple of 64; q, q_up and x 16-byte aligned.
+// CHAINS: accumulators of a warp for one output, taking turns by MMA step (two halve the chain of dependent MMAs and of f32
+// roundings).  One chain, with the epilogue rounding as gemv_mma_kernels.cuh's does (its compiler fuses scale and bias from 17
+// tokens on), gives that kernel's results bit for bit.
 // GATED: rows 0..7 of the CTA are gate rows, rows 8..15 the up rows of the same 8 channels.
-template <int NT, int KC, int W, typename YT, bool GATED, int STAGES = RingCfg<KC>::kStages>
-__global__ void __launch_bounds__((W + 1) * 32)
+template <int NT, int KC, int W, typename YT, bool GATED, int STAGES = RingCfg<KC>::kStages, int CHAINS = 2>
+__global__ void __launch_bounds__((W + 1) * 32, NT >= 3 ? 2 : 3)
 gemv_i8_ring_kernel(const int8_t *__restrict__ q, const float *__restrict__ scales, const float *__restrict__ bias,
                     const int8_t *__restrict__ q_up, const float *__restrict__ scales_up,
                     const float *__restrict__ bias_up, const uint16_t *__restrict__ x, YT *__restrict__ y, Dests extra,
@@ -162,23 +165,21 @@ gemv_i8_ring_kernel(const int8_t *__restrict__ q, const float *__restrict__ scal
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) xrow[nt] = (8 * nt + g) < M ? x + (size_t)(8 * nt + g) * K + 16 * t : nullptr;
 
-    uint4 xc[NT][2], xn[NT][2];
-#define SHREWQ_RING_LOAD_X(koff, xv)                                                              \
+    // the activations of one k-block: half h of its 16-byte pieces is read again as soon as MMA steps 2h and 2h + 1 have used it,
+    // so the next k-block's are on their way without a second set of registers
+    uint4 xc[NT][2];
+#define SHREWQ_RING_LOAD_X(koff, h)                                                               \
     _Pragma("unroll") for (int nt = 0; nt < NT; ++nt) {                                           \
-        xv[nt][0] = make_uint4(0, 0, 0, 0);                                                       \
-        xv[nt][1] = make_uint4(0, 0, 0, 0);                                                       \
-        if (xrow[nt] && (koff) < K) {                                                             \
-            xv[nt][0] = __ldg(reinterpret_cast<const uint4 *>(xrow[nt] + (koff)));                \
-            xv[nt][1] = __ldg(reinterpret_cast<const uint4 *>(xrow[nt] + (koff)) + 1);            \
-        }                                                                                         \
+        xc[nt][h] = make_uint4(0, 0, 0, 0);                                                       \
+        if (xrow[nt] && (koff) < K) xc[nt][h] = __ldg(reinterpret_cast<const uint4 *>(xrow[nt] + (koff)) + (h)); \
     }
-    SHREWQ_RING_LOAD_X(warp * 64, xc);
+    SHREWQ_RING_LOAD_X(warp * 64, 0);
+    SHREWQ_RING_LOAD_X(warp * 64, 1);
     int it = 0;
     for (int blk = blockIdx.x; blk < nblocks; blk += gridDim.x) {
-        // two accumulator sets, alternating by MMA step: halves the chain of dependent MMAs
-        float acc[2][NT][4];
+        float acc[CHAINS][NT][4];
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < CHAINS; ++h)
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -195,8 +196,7 @@ gemv_i8_ring_kernel(const int8_t *__restrict__ q, const float *__restrict__ scal
             const int k_end = K - s * KC < KC ? K - s * KC : KC;
             for (int kin = warp * 64; kin < k_end; kin += kRingWarps * 64) {
                 // this warp's next k-block (after the last one: the first of the next row block), while this one is multiplied
-                const int knext = s * KC + kin + kRingWarps * 64;
-                SHREWQ_RING_LOAD_X((knext < K ? knext : warp * 64), xn);
+                const int after = s * KC + kin + kRingWarps * 64, knext = after < K ? after : warp * 64;
                 const uint8_t *wp = stage + (size_t)g * C::kPitch + kin + 16 * t;
                 const uint4 wlo = *reinterpret_cast<const uint4 *>(wp);
                 const uint4 whi = *reinterpret_cast<const uint4 *>(wp + 8 * C::kPitch);
@@ -210,13 +210,9 @@ gemv_i8_ring_kernel(const int8_t *__restrict__ q, const float *__restrict__ scal
                     for (int nt = 0; nt < NT; ++nt) {
                         const uint4 &xa = xc[nt][j >> 1];
                         const uint32_t b0 = (j & 1) ? xa.z : xa.x, b1 = (j & 1) ? xa.w : xa.y;
-                        mma_bf16_16816(acc[j & 1][nt], a0, a1, a2, a3, b0, b1);
+                        mma_bf16_16816(acc[j & (CHAINS - 1)][nt], a0, a1, a2, a3, b0, b1);
                     }
-                }
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    xc[nt][0] = xn[nt][0];
-                    xc[nt][1] = xn[nt][1];
+                    if (j & 1) SHREWQ_RING_LOAD_X(knext, j >> 1);
                 }
             }
             __syncwarp();
@@ -227,7 +223,7 @@ gemv_i8_ring_kernel(const int8_t *__restrict__ q, const float *__restrict__ scal
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-            for (int r = 0; r < 4; ++r) s_red[warp][nt][r][lane] = acc[0][nt][r] + acc[1][nt][r];
+            for (int r = 0; r < 4; ++r) s_red[warp][nt][r][lane] = CHAINS == 2 ? acc[0][nt][r] + acc[CHAINS - 1][nt][r] : acc[0][nt][r];
         named_bar_sync(1, kRingWarps * 32);
 
         // accumulator element (lane, r) of block nt: row (lane / 4) + (r >= 2 ? 8 : 0), token 8 * nt + 2 * (lane % 4) + (r & 1)
@@ -247,15 +243,15 @@ gemv_i8_ring_kernel(const int8_t *__restrict__ q, const float *__restrict__ scal
                         gs += s_red[w][nt][mm & 1][ln];
                         us += s_red[w][nt][2 + (mm & 1)][ln];
                     }
-                    gs = gs * scales[n] + (bias ? bias[n] : 0.0f);
-                    us = us * scales_up[n] + (bias_up ? bias_up[n] : 0.0f);
+                    gs = __fadd_rn(__fmul_rn(gs, scales[n]), bias ? bias[n] : 0.0f);
+                    us = __fadd_rn(__fmul_rn(us, scales_up[n]), bias_up ? bias_up[n] : 0.0f);
                     out = gs / (1.0f + __expf(-gs)) * us;
                 } else {
                     float sum = 0.0f;
                     const int r = (mm & 1) + ((c & 8) ? 2 : 0);
 #pragma unroll
                     for (int w = 0; w < kRingWarps; ++w) sum += s_red[w][nt][r][ln];
-                    out = sum * scales[n] + (bias ? bias[n] : 0.0f);
+                    out = NT >= 3 ? __fmaf_rn(sum, scales[n], bias ? bias[n] : 0.0f) : __fadd_rn(__fmul_rn(sum, scales[n]), bias ? bias[n] : 0.0f);
                     if (epilogue == SHREWQ_EPILOGUE_RELU) out = fmaxf(out, 0.0f);
                 }
                 const size_t off = (size_t)m * ldy + n;

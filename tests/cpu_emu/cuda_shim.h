@@ -300,6 +300,9 @@ static inline void add_f32x2(float &a0, float &a1, float b0, float b1) { a0 += b
 static inline uint32_t pack_bf16x2_rn(float hi, float lo) {
     return ((uint32_t)__float2bfloat16_rn(hi).bits << 16) | __float2bfloat16_rn(lo).bits;
 }
+static inline float __fadd_rn(float a, float b) { return a + b; }
+static inline float __fmul_rn(float a, float b) { return a * b; }
+static inline float __fmaf_rn(float a, float b, float c) { return fmaf(a, b, c); }
 static inline float emu_f32_of_bf16(uint32_t bits16) { uint32_t u = bits16 << 16; float f; memcpy(&f, &u, 4); return f; }
 // (the products and sums the kernels form here are exact in f32, so one rounding to bf16 is the fused result)
 static inline uint32_t fma_bf16x2(uint32_t a, uint32_t b, uint32_t c) {

@@ -63,19 +63,20 @@ int g_ring_kc = kRingKC;
 bool g_ring_two_stages = false;
 template <int NT, int KC, typename YT, bool GATED>
 void ring_one_kc(const Args &a) {
+    constexpr int CHAINS = NT >= 3 ? 1 : 2;  // as launch_ring_m
     constexpr int NCH = GATED ? kRingRows / 2 : kRingRows;
     const unsigned grid = (unsigned)((a.N + NCH - 1) / NCH);
     if (g_ring_two_stages) {  // the launcher's choice for grids of several waves
         // (a third of the CTAs: each walks up to three row blocks through the ring)
         emu::launch((grid + 2) / 3, (kRingConsumers + 1) * 32, RingCfg<KC, 2>::kSmemBytes, [&] {
-            gemv_i8_ring_kernel<NT, KC, kRingConsumers, YT, GATED, 2>(a.q, a.scales, a.bias, a.q_up, a.scales_up, a.bias_up,
+            gemv_i8_ring_kernel<NT, KC, kRingConsumers, YT, GATED, 2, CHAINS>(a.q, a.scales, a.bias, a.q_up, a.scales_up, a.bias_up,
                                                                       static_cast<const uint16_t *>(a.x), static_cast<YT *>(a.y),
                                                                       g_peers, a.M, a.N, a.K, a.ldy, a.epilogue, &g_ring_status);
         });
         return;
     }
     emu::launch(grid, (kRingConsumers + 1) * 32, RingCfg<KC>::kSmemBytes, [&] {
-        gemv_i8_ring_kernel<NT, KC, kRingConsumers, YT, GATED>(a.q, a.scales, a.bias, a.q_up, a.scales_up, a.bias_up,
+        gemv_i8_ring_kernel<NT, KC, kRingConsumers, YT, GATED, RingCfg<KC>::kStages, CHAINS>(a.q, a.scales, a.bias, a.q_up, a.scales_up, a.bias_up,
                                                                static_cast<const uint16_t *>(a.x), static_cast<YT *>(a.y), g_peers,
                                                                a.M, a.N, a.K, a.ldy, a.epilogue, &g_ring_status);
     });
@@ -90,6 +91,7 @@ template <typename YT, bool GATED>
 void ring_m(const Args &a) {
     if (a.M <= 8) ring_one<1, YT, GATED>(a);
     else if (a.M <= 16) ring_one<2, YT, GATED>(a);
+    else if (a.M <= 24) ring_one<3, YT, GATED>(a);
     else ring_one<4, YT, GATED>(a);
 }
 

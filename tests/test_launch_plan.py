@@ -31,12 +31,13 @@ def test_small_batches_go_to_the_streaming_kernels():
         assert plan(M, 4096, 11008)[1] == "mma-ring"
         assert plan(M, 11008, 4096)[1] == "mma-ring"          # 688 CTAs: the two-stage ring
         assert plan(M, 5920, 4096, gated=1)[1] == "mma-ring"  # gated: 8 channels per CTA, 740 CTAs = five per SM
-        assert plan(M, 5928, 4096, gated=1)[1] == "mma"
-        assert plan(M, 32000, 4096)[1] == "mma"               # 2000 CTAs: the register-streaming kernel
-        assert plan(M, 4096, 4096, sms=50)[1] == "mma"
+        assert plan(M, 5928, 4096, gated=1)[1] == "mma-ring"
+        assert plan(M, 32000, 4096)[1] == "mma-ring"          # 2000 blocks of rows: a CTA walks over several
+        assert plan(M, 4096, 4096, sms=50)[1] == "mma-ring"
     for M in (17, 32):
         rc, name, p = plan(M, 4096, 4096)
-        assert (rc, name) == (0, "mma") and not any(p.values())
+        assert (rc, name) == (0, "mma-ring") and not any(p.values())
+        assert plan(M, 11008, 4096, gated=1)[1] == "mma-ring"
     assert plan(33, 4096, 4096)[1] == "tcgen05"
     assert plan(8, 4096, 4112)[1] == "tcgen05"          # the warp-MMA kernel wants in_features in blocks of 64
     assert plan(4, 4096, 4112)[1] == "gemv"
