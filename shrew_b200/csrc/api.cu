@@ -206,7 +206,8 @@ uint64_t shrewq_ctx_launch_count(const shrewq_ctx *ctx) { return ctx ? ctx->laun
 // shared memory) from 3 to 32, the tcgen05 kernel above.  The ring against warp MMA with the weights streamed through registers
 // (family "mma", by name only): at 8 tokens 4096 x 4096 6.1 against 13.0 us, gate/up 11008 x 4096 21 against 40, at 24 tokens
 // 8.1 against 11.3 and 31 against 48, with the same sums.  (tcgen05 takes 31 us there too, but in one chain per split, not eight
-// per row: its f32 results are off by 1.0e-6 against 1.2e-7, and its splits need the context's workspace.)
+// per row: its f32 results are off by 1.0e-6 against 1.2e-7, and its splits need the context's workspace.  The ring takes
+// two tokens of that pair in 20 us against the GEMV's 25, but in chains of MMAs instead of fused multiply-adds.)
 // f32 activations on SMALL layers (config 1: 784 -> 256 -> 10 at 64 tokens): the whole forward is a few MFLOP and
 // what counts is the number and latency of launches; the CUDA-core GEMV in slices of tokens is one short launch
 // where the tensor-core route never fills (and it keeps every bit of x, which the hi/lo pair does not).
@@ -214,12 +215,7 @@ constexpr size_t kGemvSlicedMaxTokens = 128;
 static bool gemv_slices_win(size_t M, size_t N, size_t K) {
     return M > 16 && M <= kGemvSlicedMaxTokens && M * N * K <= ((size_t)1 << 26);
 }
-// Two tokens on large weights with bf16 results: the ring kernel (25.6 -> 20.4 us on the gate/up pair 11008 x 4096).
-static bool two_tokens_on_ring(size_t M, size_t N, size_t K, bool gated, bool y_bf16) {
-    return M == 2 && y_bf16 && N * K * (gated ? 2 : 1) >= ((size_t)1 << 25);
-}
-static int default_family(size_t M, size_t N, size_t K, bool gated, bool y_bf16, bool gemv_ok, bool mma_ok, bool tc_ok) {
-    if (mma_ok && two_tokens_on_ring(M, N, K, gated, y_bf16)) return kForceRing;
+static int default_family(size_t M, bool gemv_ok, bool mma_ok, bool tc_ok) {
     if (gemv_ok && (M <= 2 || (!mma_ok && (M <= 4 || !tc_ok)))) return kForceGemv;
     if (mma_ok && M <= 32) return kForceRing;
     return tc_ok ? kForceTc : (gemv_ok ? kForceGemv : kForceSimt);
@@ -247,7 +243,7 @@ int shrewq_plan_forward(size_t M, size_t N, size_t K, int x_is_bf16, int gated, 
     const bool small = M < (1u << 31) && N < (1u << 31) && K < (1u << 31);
     const bool tc_ok = x_is_bf16 && vec16 && M >= 1 && small;
     const bool mma_ok = x_is_bf16 && (K % 64) == 0 && M <= 64 && small;
-    int fam = default_family(M, N, K, gated != 0, false, vec16 && M <= 16, mma_ok, tc_ok);
+    int fam = default_family(M, vec16 && M <= 16, mma_ok, tc_ok);
     if (!x_is_bf16 && vec16 && small && M > 16 && !gated) fam = kForceTcF32;   // f32 activations: the hi/lo tensor-core pass
     if (!x_is_bf16 && vec16 && small && gemv_slices_win(M, N, K)) fam = kForceGemv;
     if (fam == kForceTc && M > 128 && pair_kernel_wins(M, N, K, gated != 0)) fam = kForceTc2Cta;
@@ -687,7 +683,7 @@ static int forward_impl(shrewq_linear *lin, shrewq_linear *up, const void *x_dev
             } else if (M > 128 && tc_ok && (ctx->tuning.tc_pair == 2 || (ctx->tuning.tc_pair == 1 && pair_kernel_wins(M, lin->n, lin->k, up != nullptr)))) {
                 choice = kForceTc2Cta;
             } else {
-                choice = default_family(M, lin->n, lin->k, up != nullptr, a.y_dtype == SHREWQ_BF16, gemv_ok, mma_ok, tc_ok);
+                choice = default_family(M, gemv_ok, mma_ok, tc_ok);
             }
     }
     const char *name;

@@ -21,8 +21,10 @@ def _x(M, K):
     return torch.randn((M, K), device="cuda", generator=torch.Generator(device="cuda").manual_seed(M)).to(torch.bfloat16)
 
 
-# CTA pairs whose tiles are split along K (16 channel pairs, K = 11008): four ways at 200 tokens, two ways up to 512; 17 to 32 tokens on weights from 2^25 codes on
-@pytest.mark.parametrize("M,N,K", [(200, 4096, 11008), (384, 4096, 11008), (512, 4096, 11008), (17, 11008, 4096), (32, 4096, 11008)])
+# CTA pairs whose tiles are split along K (16 channel pairs, K = 11008): four ways at 200 tokens, two ways up to 512; 17 to 32 and two
+# tokens on weights from 2^25 codes on
+@pytest.mark.parametrize("M,N,K", [(200, 4096, 11008), (384, 4096, 11008), (512, 4096, 11008), (17, 11008, 4096), (32, 4096, 11008),
+                                   (2, 11008, 4096), (2, 4096, 11008)])
 def test_bf16_result_is_the_rounded_f32_result(M, N, K):
     ql, x = _layer(N, K, N + K), _x(M, K)
     assert torch.equal(ql.forward(x), ql.forward(x, out_dtype=torch.float32).to(torch.bfloat16))
