@@ -100,12 +100,14 @@ int launch_ring_one(shrewq_ctx *ctx, const ForwardArgs &a) {
     }
 }
 
-// Chains of a warp's sums: two up to 16 tokens; one above, which are the sums (bit for bit) of the register-streaming kernel
-// that ran these calls before.
+// Chains of a warp's sums: two up to 16 tokens on grids of up to five CTAs per SM; one on larger grids and above 16 tokens, which
+// are the sums (bit for bit) of the register-streaming kernel that ran these calls before.  One chain costs 3 % up to
+// 8 tokens: gate/up 11008 x 4096 at 3 tokens 20.4 -> 21.0 us.
 template <typename YT, bool GATED>
 int launch_ring_m(shrewq_ctx *ctx, const ForwardArgs &a) {
-    if (a.M <= 8) return launch_ring_one<1, 2, YT, GATED>(ctx, a);
-    if (a.M <= 16) return launch_ring_one<2, 2, YT, GATED>(ctx, a);
+    const bool one = (a.N + (GATED ? 7 : 15)) / (GATED ? 8 : 16) > (size_t)5 * ctx->sm_count;
+    if (a.M <= 8) return one ? launch_ring_one<1, 1, YT, GATED>(ctx, a) : launch_ring_one<1, 2, YT, GATED>(ctx, a);
+    if (a.M <= 16) return one ? launch_ring_one<2, 1, YT, GATED>(ctx, a) : launch_ring_one<2, 2, YT, GATED>(ctx, a);
     if (a.M <= 24) return launch_ring_one<3, 1, YT, GATED>(ctx, a);
     return launch_ring_one<4, 1, YT, GATED>(ctx, a);
 }

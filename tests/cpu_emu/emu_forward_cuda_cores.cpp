@@ -61,9 +61,12 @@ void gemv_g(const Args &a) {
 DeviceStatus g_ring_status{};
 int g_ring_kc = kRingKC;
 bool g_ring_two_stages = false;
-template <int NT, int KC, typename YT, bool GATED>
+template <int NT, int KC, typename YT, bool GATED, int CHAINS = 1>
 void ring_one_kc(const Args &a) {
-    constexpr int CHAINS = NT >= 3 ? 1 : 2;  // as launch_ring_m
+    // as launch_ring_m (here two stages, the larger grids, go with one chain)
+    if constexpr (NT < 3 && CHAINS == 1) {
+        if (!g_ring_two_stages) return ring_one_kc<NT, KC, YT, GATED, 2>(a);
+    }
     constexpr int NCH = GATED ? kRingRows / 2 : kRingRows;
     const unsigned grid = (unsigned)((a.N + NCH - 1) / NCH);
     if (g_ring_two_stages) {  // the launcher's choice for grids of several waves

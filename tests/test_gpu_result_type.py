@@ -62,6 +62,20 @@ def test_17_to_32_tokens_of_a_gated_pair(M, N, K):
         assert torch.equal(*out)
 
 
+# Up to 16 tokens the same holds from more than five CTAs of 16 rows per SM on
+@pytest.mark.parametrize("M,rows_per_sm,gated", [(3, 81, False), (8, 200, False), (16, 81, False), (9, 41, True), (16, 75, True)])
+def test_large_grids_are_summed_as_by_the_register_streaming_kernel(M, rows_per_sm, gated):
+    N = rows_per_sm * torch.cuda.get_device_properties(0).multi_processor_count
+    gate, x = _layer(N, 2176, 5, True), _x(M, 2176)
+    up = _layer(N, 2176, 6) if gated else None
+    for dtype in (torch.float32, torch.bfloat16):
+        out = [torch.empty((M, N), dtype=dtype, device="cuda") for _ in range(2)]
+        for y, kind in zip(out, ("auto", "mma")):
+            _run(kind, lambda: gate.forward_gate_up_silu(up, x, out=y) if gated else gate.forward(x, out=y))
+            assert gate.last_kernel() == ("mma" if kind == "mma" else "mma-ring")
+        assert torch.equal(*out)
+
+
 # These calls need no workspace of the context: the first one of a new context can be captured, and calls on two streams share
 # nothing.
 @pytest.mark.parametrize("M", [24, 64])
