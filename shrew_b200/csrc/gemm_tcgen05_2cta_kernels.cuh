@@ -224,6 +224,9 @@ linear_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const 
                                        ((uint32_t)((2 * kLanes) >> 4) << 24);
             const uint64_t bdesc0 = make_b_desc(smem_base + kXOff);
             const uint32_t a0 = tmem_base + kABase;
+            // the activations come after the previous kernel, however long that takes (a barrier between GPUs tolerates a
+            // late peer): the time limit of the waits starts when it has completed
+            pdl_wait();
             uint32_t s = 0, ph = 0, a_tmem = a0;
             uint64_t bdesc = bdesc0;
             bool ok = true;
@@ -268,6 +271,7 @@ linear_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const 
             const int s = i % kStages;
             if (s % kGroups != group) continue;
             const uint32_t ph = (i / kStages) & 1;
+            if (ph == 1) pdl_wait();  // a stage is refilled after its first MMA, which waits for the previous kernel
             if (quad == 0) TRACE2(2, i, 0);
             ok = mbar_wait_warp(bars_u32 + kWFull + s * 8, ph, ctl, status, 3, s);
             if (!ok) break;

@@ -134,6 +134,7 @@ linear_i8_tcgen05_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const f
                 const int n0 = (tile % n_tiles) * kF32Chan;
                 for (int kb = 0; kb < nkb; ++kb, ++it) {
                     const int s = it % C::kWStages;
+                    if (it == C::kWStages) pdl_wait();  // (below)
                     if (it >= C::kWStages) ok = f32_wait(bars + C::kWEmpty + 8 * s, ((it / C::kWStages) - 1) & 1, ctl, status, 0, s);
                     if (!ok) break;
                     mbar_expect_tx(bars + C::kWFull + 8 * s, C::kWBytes);
@@ -147,6 +148,7 @@ linear_i8_tcgen05_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const f
         if (elect_one()) {
             // D=f32, A=bf16 (K-major, tensor memory), B=bf16 (K-major), M=128, N=TOK
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TOK >> 3) << 17) | ((uint32_t)(kF32Chan >> 4) << 24);
+            pdl_wait();  // the first activations come after it: a time limit must not run while the previous kernel does
             int it = 0, li = 0, visit_load = 0;  // visit_load: index of the first activation block of this token tile
             bool ok = true;
             for (int tile = begin; tile < end && ok; ++tile, ++li) {
@@ -183,6 +185,9 @@ linear_i8_tcgen05_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const f
         const int total = (end - begin) * nkb;
         for (int it = (warp - 2) >> 2; it < total; it += 2) {
             const int s = it % C::kWStages, as = it % C::kAStages;
+            // as far as the free stages reach the codes are widened while the previous kernel still runs
+            constexpr int kFree = C::kWStages < C::kAStages ? C::kWStages : C::kAStages;
+            if (it == kFree || it == kFree + 1) pdl_wait();
             if (!f32_wait_warp(bars + C::kWFull + 8 * s, (it / C::kWStages) & 1, ctl, status, 4, s)) break;
             uint32_t packed[32];
             convert_row64(smem + C::kWOff + s * C::kWBytes + row * kF32BlockK, swz, packed);

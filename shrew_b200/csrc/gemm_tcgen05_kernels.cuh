@@ -225,6 +225,7 @@ linear_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
                                        ((uint32_t)(TOK >> 3) << 17) | ((uint32_t)(kTileN >> 4) << 24);
             const uint64_t bdesc0 = make_b_desc(smem_base + C::kXOff);
             const uint32_t a0 = tmem_base + C::kABase;
+            pdl_wait();  // (as the converters)
             uint32_t s = 0, ph = 0, a_tmem = a0;
             uint64_t bdesc = bdesc0;
             bool ok = true;
@@ -273,6 +274,9 @@ linear_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
         // A group owns pipeline STAGES (stage s belongs to group s % G), not every G-th round: its
         // warps then pass through every phase of the barriers they poll, so a parity wait can never
         // mistake phase k-2 for phase k, whatever order the TMA loads complete in.
+        // A stage is full only with its activations, which come after the previous kernel, however long that takes (a
+        // barrier between GPUs tolerates a late peer): the time limit of the waits starts when it has completed.
+        pdl_wait();
         for (int i = 0; i < nr && ok; ++i) {
             const int s = i % C::kStages;
             if (s % G != group) continue;
@@ -296,7 +300,7 @@ linear_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
             if (((warp - 2) & 3) == 0) TRACE(2, i, 3);
         }
         // ---------------- epilogue: 16-column chunks dealt round-robin to the groups ----------------
-        pdl_wait();  // outputs, partial sums and counters may still be in use by the previous kernel of the stream
+        // (after pdl_wait: outputs, partial sums and counters may be in use by the previous kernel of the stream)
         if (warp == 2) TRACE(3, 0, 0);  // (tracing build: role 3 = the epilogue of the first converter warp)
         if (ok) ok = mbar_wait_warp(bars_u32 + kAccBar, 0, ctl, status, 4, 0);
         if (warp == 2) TRACE(3, 0, 1);  // accumulators complete

@@ -32,7 +32,7 @@
 // before they read activations or write outputs.  A chain of small-batch forwards thus keeps the weight stream
 // going across kernel boundaries.  Launched without the attribute the two instructions do nothing.
 //
-// Every wait is bounded: a wait that runs out records itself in DeviceStatus (timeout code 4) and the CTA
+// Every wait is bounded, and none that depends on the consumers starts before the previous kernel has completed: a wait that runs out records itself in DeviceStatus (timeout code 4) and the CTA
 // leaves without writing.
 //
 // Device code only (PTX behind ptx_small.cuh / ptx_tcgen05.cuh): also compiles against the CUDA stand-in of the
@@ -50,7 +50,10 @@ namespace {
 
 // W consumer warps (8 or 16) + one producer warp (warp W)
 constexpr int kRingRows = 16;                          // rows of W per CTA
-constexpr uint32_t kRingSpinLimit = 1u << 22;          // bounded wait: a few tenths of a second with the pauses
+#ifndef SHREWQ_RING_SPIN_LIMIT
+#define SHREWQ_RING_SPIN_LIMIT (1u << 22)
+#endif
+constexpr uint32_t kRingSpinLimit = SHREWQ_RING_SPIN_LIMIT;  // bounded wait: a few tenths of a second with the pauses
 constexpr unsigned int kTimeoutRing = 4;               // DeviceStatus::timeout_flag of this kernel
 
 // KC: bytes (= codes) of k per row and stage, i.e. the size of one bulk copy.  The copy engine's cost is per copy:
@@ -142,6 +145,9 @@ gemv_i8_ring_kernel(const int8_t *__restrict__ q, const float *__restrict__ scal
             for (int s = 0; s < nstages; ++s, ++it) {
                 const int slot = it % S;
                 if (it >= S) {
+                    // the consumers free a slot only after their own wait for the previous kernel, however long that takes
+                    // (a barrier between GPUs tolerates a late peer): the time limit starts when it has completed
+                    if (it == S) pdl_wait();
                     int good = 1;
                     if (lane == 0) good = ring_wait(empty_u32 + slot * 8, ((it / S) - 1) & 1, status, 1, s) ? 1 : 0;
                     ok = __shfl_sync(0xFFFFFFFFu, good, 0) != 0;

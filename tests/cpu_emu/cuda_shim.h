@@ -295,7 +295,15 @@ static inline float __fdividef(float a, float b) { return a / b; }
 static inline uint4 ld_stream_16(const void *p) { uint4 v; memcpy(&v, p, 16); return v; }
 static inline float ld_cg_ordered(const float *p) { return *p; }
 static inline void pdl_launch_dependents() {}   // launches are sequential here
-static inline void pdl_wait() {}
+// Programmatic dependent launch: the previous kernel of the stream completes at this time of the steady clock
+namespace emu { inline std::atomic<long long> g_predecessor_ends_us{0}; }
+static inline void pdl_wait() {
+    auto now = [] { return std::chrono::duration_cast<std::chrono::microseconds>(std::chrono::steady_clock::now().time_since_epoch()).count(); };
+    while (now() < emu::g_predecessor_ends_us.load()) std::this_thread::sleep_for(std::chrono::milliseconds(2));
+}
+extern "C" inline __attribute__((used, visibility("default"))) void emu_predecessor_ends_in_ms(int ms) {
+    emu::g_predecessor_ends_us = std::chrono::duration_cast<std::chrono::microseconds>(std::chrono::steady_clock::now().time_since_epoch()).count() + 1000ll * ms;
+}
 static inline void add_f32x2(float &a0, float &a1, float b0, float b1) { a0 += b0; a1 += b1; }
 static inline uint32_t pack_bf16x2_rn(float hi, float lo) {
     return ((uint32_t)__float2bfloat16_rn(hi).bits << 16) | __float2bfloat16_rn(lo).bits;

@@ -827,17 +827,48 @@ def test_cta_pair_tile_list_and_tail_split(oracle, emu_pair, gated):
 # TMA load is dropped on purpose (host-side injection, nothing faults) and the kernel, compiled with small
 # wait limits (so small that other roles give up at about the same time, wherever they happen to be), has
 # to return with the status set while its 448 threads sit in barriers of every kind.
-def _build_short_waits(name):
+def _build_short_waits(name, limits=("-DSHREWQ_SPIN_FAST_LIMIT=64", "-DSHREWQ_SPIN_SLOW_LIMIT=40"), suffix="short_waits"):
     src = os.path.join(EMU_DIR, name + ".cpp")
-    out = os.path.join(BUILD_DIR, "lib" + name + "_short_waits.so")
+    out = os.path.join(BUILD_DIR, f"lib{name}_{suffix}.so")
     os.makedirs(BUILD_DIR, exist_ok=True)
     deps = [src] + [os.path.join(ROOT, "shrew_b200", "csrc", h) for h in os.listdir(os.path.join(ROOT, "shrew_b200", "csrc")) if h.endswith(".cuh")] + [
         os.path.join(EMU_DIR, h) for h in os.listdir(EMU_DIR) if h.endswith(".h")]
     if not os.path.exists(out) or any(os.path.getmtime(d) > os.path.getmtime(out) for d in deps):
         subprocess.run(["g++", "-std=c++20", "-O1", "-pthread", "-fPIC", "-shared", "-ffp-contract=off", "-fno-fast-math",
-                        "-Wno-unknown-pragmas", "-DSHREWQ_SPIN_FAST_LIMIT=64", "-DSHREWQ_SPIN_SLOW_LIMIT=40", "-o", out, src],
+                        "-Wno-unknown-pragmas", *limits, "-o", out, src],
                        check=True, cwd=EMU_DIR)
     return ctypes.CDLL(out)
+
+
+# Programmatic dependent launch: the kernel starts while the previous one (a barrier between GPUs, say) still runs, here for four
+# seconds, and no wait, all limited to about one second, may run out because of it.  Shapes in which every ring wraps.
+@pytest.mark.parametrize("kernel", ["ring", "f32", "tcgen05", "pair"])
+@pytest.mark.timeout(300)
+def test_no_wait_runs_out_while_the_previous_kernel_runs(oracle, kernel):
+    limits = ("-DSHREWQ_SPIN_FAST_LIMIT=64", "-DSHREWQ_SPIN_SLOW_LIMIT=10000", "-DSHREWQ_RING_SPIN_LIMIT=10000")
+    name = {"ring": "emu_forward_cuda_cores", "f32": "emu_gemm_tcgen05_f32", "tcgen05": "emu_gemm_tcgen05", "pair": "emu_gemm_tcgen05_pair"}[kernel]
+    L = _build_short_waits(name, limits, "second_waits")
+    M, N, K = {"ring": (20, 33, 64 * 170), "f32": (70, 300, 832), "tcgen05": (20, 128, 2048), "pair": (256, 256, 1024)}[kernel]
+    q, scales, bias, x_bits, x = _tc_case(M, N, K, 3)
+    ref = oracle.np_linear_forward(q, scales, oracle.PER_CHANNEL, bias, x)
+    qa, xa, y, s32 = _aligned(q.shape, np.int8), _aligned(x_bits.shape, np.float32 if kernel == "f32" else np.uint16), np.zeros((M, N), np.float32), scales.astype(np.float32)
+    qa[...], xa[...] = q, x if kernel == "f32" else x_bits
+    L.emu_predecessor_ends_in_ms(4000)
+    if kernel == "ring":
+        L.emu_forward_cuda_cores.argtypes = [_ci, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ci, _ci, _ci, _sz, _ci, _ci, _ci, _ci]
+        L.emu_set_ring_two_stages(1)
+        rc = L.emu_forward_cuda_cores(2, _p(qa), _p(s32), _p(bias), None, None, None, _p(xa), _p(y), M, N, K, N, 0, 1, 0, 1)
+    elif kernel == "f32":
+        L.emu_gemm_tcgen05_f32.argtypes = [_vp, _vp, _vp, _vp, _vp, _ci, _ci, _ci, _sz, _ci, _ci, _ci]
+        rc = L.emu_gemm_tcgen05_f32(_p(qa), _p(s32), _p(bias), _p(xa), _p(y), M, N, K, N, 0, 64, 1)
+    elif kernel == "tcgen05":
+        L.emu_gemm_tcgen05.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ci, _ci, _ci, _sz, _ci, _ci, _ci, _ci, _ci, _ci]
+        rc = L.emu_gemm_tcgen05(_p(qa), _p(s32), _p(bias), None, None, None, _p(xa), _p(y), M, N, K, N, 0, 0, 32, 3, 1, 0)
+    else:
+        L.emu_gemm_tcgen05_pair.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ci, _ci, _ci, _sz, _ci, _ci, _ci, _ci]
+        rc = L.emu_gemm_tcgen05_pair(_p(qa), _p(s32), _p(bias), None, None, None, _p(xa), _p(y), M, N, K, N, 0, 0, 1, 0)
+    assert rc == 0
+    assert oracle.rel_err(y, ref) < (1e-4 if kernel == "f32" else 2e-5)
 
 
 @pytest.mark.parametrize("tok,M,N,K,splits,gated,drop", [
