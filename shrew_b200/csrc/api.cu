@@ -112,9 +112,14 @@ int shrewq_ctx_create(int device, void *stream, shrewq_ctx **out) {
     ctx->stream = static_cast<cudaStream_t>(stream);
     ctx->sm_count = prop.multiProcessorCount;
     if (cudaSetDevice(device) != cudaSuccess || cudaMalloc(&ctx->dev_status, sizeof(DeviceStatus)) != cudaSuccess ||
-        cudaMemset(ctx->dev_status, 0, sizeof(DeviceStatus)) != cudaSuccess) {
+        cudaMemset(ctx->dev_status, 0, sizeof(DeviceStatus)) != cudaSuccess ||
+        cudaMalloc(&ctx->tensor_slots, kTensorSlots * kTensorSlotBytes) != cudaSuccess ||
+        cudaMemset(ctx->tensor_slots, 0, kTensorSlots * kTensorSlotBytes) != cudaSuccess ||
+        cudaStreamSynchronize(nullptr) != cudaSuccess) {
         int rc = set_err(nullptr, SHREWQ_ERR_CUDA, "ctx_create: device setup failed: %s",
                          cudaGetErrorString(cudaGetLastError()));
+        if (ctx->tensor_slots) cudaFree(ctx->tensor_slots);
+        if (ctx->dev_status) cudaFree(ctx->dev_status);
         delete ctx;
         return rc;
     }
@@ -177,6 +182,7 @@ void shrewq_ctx_destroy(shrewq_ctx *ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     if (ctx->scratch) cudaFree(ctx->scratch);
+    if (ctx->tensor_slots) cudaFree(ctx->tensor_slots);
     if (ctx->stage_dev) cudaFree(ctx->stage_dev);
     if (ctx->xsplit) cudaFree(ctx->xsplit);
     if (ctx->ytmp) cudaFree(ctx->ytmp);

@@ -17,6 +17,7 @@
 namespace shrewq {
 
 constexpr int kErrLen = 512;
+constexpr size_t kTensorSlotBytes = 16640, kTensorSlots = 8;
 
 // Launch options of a context (shrewq_ctx_set_option); the defaults are the measured choices.
 struct Tuning {
@@ -41,9 +42,14 @@ struct shrewq_ctx {
     char err[shrewq::kErrLen] = {0};
     std::atomic<uint64_t> launches{0};
     shrewq::Tuning tuning;
-    // scratch: quantizer words, split-K tile counters (both zeroed with the allocation, left at zero by the kernels), partial sums
+    // scratch: words of the other quantizers, split-K tile counters (both zeroed with the allocation, left at zero by the kernels), partial sums
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
+    // per-tensor quantization (parameters, partial extrema, arrival counter of one call): memory of its own, allocated and
+    // zeroed with the context, so that a quantize on one stream does not meet a split-K forward on another and needs nothing
+    // under capture.  Calls take the slots in turn: so many may be in flight on different streams.
+    void *tensor_slots = nullptr;
+    std::atomic<unsigned int> tensor_calls{0};
     // the gated block's host-buffer entry point: two staging slots and two copy streams, so that the copies of
     // one call overlap the kernels of its neighbours (created on first use)
     cudaStream_t copy_in = nullptr, copy_out = nullptr;

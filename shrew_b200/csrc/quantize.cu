@@ -59,16 +59,14 @@ bool rows_in_registers(shrewq_ctx *ctx, const T *w, size_t rows, size_t cols, in
 // Per-tensor in two launches (extrema and parameters, codes), the second one allowed to start under the first one's tail.
 template <typename T, bool ASYM>
 int tensor_two_pass(shrewq_ctx *ctx, const T *w, size_t n, int bits, int8_t *q, double *scales, double *zps) {
-    // scratch: the arrival counter in the head that is zeroed with the allocation, the rest where split-K keeps partial sums
-    int rc = ensure_scratch(ctx, 8192 + sizeof(TensorGroup));
-    if (rc != SHREWQ_OK) return rc;
-    unsigned int *arrived = reinterpret_cast<unsigned int *>(static_cast<char *>(ctx->scratch) + 4032);
-    TensorGroup *g = reinterpret_cast<TensorGroup *>(static_cast<char *>(ctx->scratch) + 8192);
+    static_assert(sizeof(TensorGroup) <= kTensorSlotBytes && kTensorSlotBytes % 64 == 0, "a slot holds one call's words");
+    TensorGroup *g = reinterpret_cast<TensorGroup *>(static_cast<char *>(ctx->tensor_slots) +
+                                                     ctx->tensor_calls.fetch_add(1, std::memory_order_relaxed) % kTensorSlots * kTensorSlotBytes);
     const size_t vecs = n / Vec16<T>::kElems;
     const size_t cap = (size_t)ctx->sm_count * 8 < (size_t)kMaxPartials ? (size_t)ctx->sm_count * 8 : (size_t)kMaxPartials;
     const size_t want = (vecs + 1023) / 1024;
     SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(extrema_partials_kernel<T, ASYM>, dim3((unsigned)(want < 1 ? 1 : (want > cap ? cap : want))), dim3(256), 0,
-                                          ctx->stream, true, w, n, bits, g, arrived, scales, zps));
+                                          ctx->stream, true, w, n, bits, g, scales, zps));
     ctx->launches += 1;
     if (n > 0) {
         constexpr int U = sizeof(T) == 2 ? 2 : 4;

@@ -289,6 +289,7 @@ constexpr int kMaxPartials = 2048;
 struct TensorGroup {
     GroupParams p;
     FastGroup f;
+    unsigned int arrived;
     alignas(16) Extrema partials[kMaxPartials];  // read as float2
 };
 static_assert(sizeof(Extrema) == 8, "an Extrema is two floats");
@@ -296,7 +297,7 @@ static_assert(sizeof(Extrema) == 8, "an Extrema is two floats");
 #ifndef SHREWQ_CPU_EMU  // (the CPU model has no wrapping atomic)
 template <typename T, bool ASYM>
 __global__ void __launch_bounds__(256)
-extrema_partials_kernel(const T *__restrict__ w, size_t n, int bits, TensorGroup *g, unsigned int *arrived, double *__restrict__ scales,
+extrema_partials_kernel(const T *__restrict__ w, size_t n, int bits, TensorGroup *g, double *__restrict__ scales,
                         double *__restrict__ zps) {
     // in this order: the second launch reads w before its own wait, so none of it may start before w is complete
     pdl_wait();
@@ -322,7 +323,7 @@ extrema_partials_kernel(const T *__restrict__ w, size_t n, int bits, TensorGroup
     if (threadIdx.x == 0) {
         g->partials[blockIdx.x] = e;
         __threadfence();
-        s_last = atomicInc(arrived, gridDim.x - 1) == gridDim.x - 1;
+        s_last = atomicInc(&g->arrived, gridDim.x - 1) == gridDim.x - 1;
     }
     __syncthreads();
     if (!s_last) return;
