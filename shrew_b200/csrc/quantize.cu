@@ -71,7 +71,7 @@ int tensor_two_pass(shrewq_ctx *ctx, const T *w, size_t n, int bits, int8_t *q, 
     if (n > 0) {
         constexpr int U = sizeof(T) == 2 ? 2 : 4;
         SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(quantize_tensor_kernel<T, ASYM, U>, dim3((unsigned)(want < 1 ? 1 : (vecs + 256 * U - 1) / (256 * U))),
-                                              dim3(256), 0, ctx->stream, true, w, n, static_cast<const TensorGroup *>(g), q));
+                                              dim3(256), 0, ctx->stream, true, w, n, g, q));
         ctx->launches += 1;
     }
     return SHREWQ_OK;

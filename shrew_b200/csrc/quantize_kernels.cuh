@@ -281,8 +281,8 @@ absmax_flat_kernel(const float *__restrict__ w, size_t n, unsigned int *amax_bit
 }
 
 // Per-tensor in two launches.  Every block leaves the extrema of its contiguous part; the block that finishes last
-// reduces them and forms the tensor's parameters, so no kernel of one thread sits between the passes and nothing has
-// to be cleared (the counter wraps to zero by itself).  The second pass takes the tensor from its end, where the
+// reduces them and forms the tensor's parameters, so no kernel of one thread sits between the passes.  The second pass leaves the
+// counter at zero for the slot's next call, whatever calls that overlapped on other streams made of it.  The second pass takes the tensor from its end, where the
 // first one stopped: that much of it may still be in L2.
 constexpr int kMaxPartials = 2048;
 
@@ -294,7 +294,6 @@ struct TensorGroup {
 };
 static_assert(sizeof(Extrema) == 8, "an Extrema is two floats");
 
-#ifndef SHREWQ_CPU_EMU  // (the CPU model has no wrapping atomic)
 template <typename T, bool ASYM>
 __global__ void __launch_bounds__(256)
 extrema_partials_kernel(const T *__restrict__ w, size_t n, int bits, TensorGroup *g, double *__restrict__ scales,
@@ -323,7 +322,7 @@ extrema_partials_kernel(const T *__restrict__ w, size_t n, int bits, TensorGroup
     if (threadIdx.x == 0) {
         g->partials[blockIdx.x] = e;
         __threadfence();
-        s_last = atomicInc(&g->arrived, gridDim.x - 1) == gridDim.x - 1;
+        s_last = gridDim.x == 1 || atomicAdd(&g->arrived, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!s_last) return;
@@ -347,7 +346,7 @@ extrema_partials_kernel(const T *__restrict__ w, size_t n, int bits, TensorGroup
 // 256 * U consecutive vectors.
 template <typename T, bool ASYM, int U>
 __global__ void __launch_bounds__(256)
-quantize_tensor_kernel(const T *__restrict__ w, size_t n, const TensorGroup *g, int8_t *__restrict__ q) {
+quantize_tensor_kernel(const T *__restrict__ w, size_t n, TensorGroup *g, int8_t *__restrict__ q) {
     pdl_launch_dependents();
     constexpr int EPV = Vec16<T>::kElems;
     const bool aligned = ((reinterpret_cast<uintptr_t>(w) & 15) == 0) && ((reinterpret_cast<uintptr_t>(q) & (EPV - 1)) == 0);
@@ -358,6 +357,7 @@ quantize_tensor_kernel(const T *__restrict__ w, size_t n, const TensorGroup *g, 
 #pragma unroll
     for (int u = 0; u < U; ++u) r[u] = first + u * 256 < nvec ? __ldcs(w4 + first + u * 256) : make_uint4(0, 0, 0, 0);
     pdl_wait();
+    if (blockIdx.x == 0 && threadIdx.x == 0) g->arrived = 0;
     const FastGroup f = g->f;
     const uint32_t all = f.exact ? (1u << EPV) - 1u : 0u;
 #pragma unroll
@@ -381,7 +381,6 @@ quantize_tensor_kernel(const T *__restrict__ w, size_t n, const TensorGroup *g, 
         q[j] = all || undecided<ASYM>(d) ? (int8_t)quant_ex(widen(w[j]), g->p) : (int8_t)m;
     }
 }
-#endif  // SHREWQ_CPU_EMU
 
 struct TensorParams {
     RowParams p;

@@ -47,6 +47,7 @@ struct uint2 { uint32_t x, y; };
 struct uint4 { unsigned x, y, z, w; };
 static inline float4 make_float4(float x, float y, float z, float w) { return float4{x, y, z, w}; }
 static inline uint4 make_uint4(unsigned x, unsigned y, unsigned z, unsigned w) { return uint4{x, y, z, w}; }
+struct float2 { float x, y; };
 
 namespace emu {
 // A violated rule of the model (more arrivals than a barrier expects, a tensor-memory access outside the

@@ -43,7 +43,24 @@ extern "C" int emu_quantize_rows(const float *w, size_t rows, size_t cols, int v
     return 0;
 }
 
-// the per-tensor chain of launch_quantize: amax with atomics, parameters, element map
+// Per-tensor in two launches as tensor_two_pass: partial extrema, codes.  arrived: what the slot's counter holds before and after.
+extern "C" int emu_quantize_tensor_two_pass(const float *w, size_t n, int bits, int asym, unsigned grid, unsigned *arrived, int8_t *q, double *scale,
+                                            double *zp) {
+    auto g = std::make_unique<TensorGroup>();
+    g->arrived = *arrived;
+    const unsigned blocks = std::max<unsigned>(1, (unsigned)((n / 4 + 1023) / 1024));
+    if (asym) {
+        emu::launch(grid, 256, [&] { extrema_partials_kernel<float, true>(w, n, bits, g.get(), scale, zp); });
+        if (n) emu::launch(blocks, 256, [&] { quantize_tensor_kernel<float, true, 4>(w, n, g.get(), q); });
+    } else {
+        emu::launch(grid, 256, [&] { extrema_partials_kernel<float, false>(w, n, bits, g.get(), scale, zp); });
+        if (n) emu::launch(blocks, 256, [&] { quantize_tensor_kernel<float, false, 4>(w, n, g.get(), q); });
+    }
+    *arrived = g->arrived;
+    return 0;
+}
+
+// the per-tensor chain from a supplied or reduced amax: amax with atomics, parameters, element map
 extern "C" int emu_quantize_tensor(const float *w, size_t n, unsigned grid, int8_t *q, double *scale) {
     alignas(16) unsigned char scratch[256] = {0};
     unsigned int *amax_bits = reinterpret_cast<unsigned int *>(scratch);
