@@ -12,6 +12,7 @@
 #include <Python.h>
 
 #include <ATen/cuda/EmptyTensor.h>
+#include <ATen/cuda/PeerToPeerAccess.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/DynamicTypes.h>
 #include <torch/csrc/Dtype.h>
@@ -33,7 +34,6 @@ struct Library {
     decltype(&shrewq_quantize_f32_ex) quantize_f32_ex = nullptr;
     decltype(&shrewq_quantize_any) quantize_any = nullptr;
     decltype(&shrewq_quantize_f32_batch) quantize_f32_batch = nullptr;
-    decltype(&shrewq_dequantize) dequantize = nullptr;
     decltype(&shrewq_dequantize_ex) dequantize_ex = nullptr;
     decltype(&shrewq_linear_forward) linear_forward = nullptr;
     decltype(&shrewq_linear_forward_gate_up_silu) gate_up_silu = nullptr;
@@ -172,16 +172,19 @@ at::Tensor checked_output(const Layer *l, PyObject *out, int64_t M, at::ScalarTy
         return empty(shape, type, l->device);
     }
     const at::Tensor &y = tensor_arg(out, who);
+    // (another GPU's memory may be written where the two have peer access)
+    if (y.numel() > 0 && (!y.is_cuda() || (y.get_device() != l->device && !at::cuda::get_p2p_access((c10::DeviceIndex)l->device, (c10::DeviceIndex)y.get_device()))))
+        fail(SHREWQ_ERR_INVALID_ARG, std::string(who) + ": the output buffer is not on the layer's device");
     if (y.dim() != 2 || y.size(0) != M || y.size(1) != l->out_features || (M > 0 && y.stride(1) != 1) || act_code(y.scalar_type()) < 0)
         fail(SHREWQ_ERR_INVALID_ARG, std::string(who) + ": bad output buffer");
     *ldy = (size_t)(M > 1 ? y.stride(0) : std::max(y.stride(0), l->out_features));
     return y;
 }
 
-at::ScalarType dtype_arg(PyObject *o, at::ScalarType otherwise) {
+at::ScalarType dtype_arg(PyObject *o, at::ScalarType otherwise, const char *what) {
     if (!o || o == Py_None) return otherwise;
     if (!THPDtype_Check(o)) {
-        PyErr_SetString(PyExc_TypeError, "forward: out_dtype is a torch.dtype");
+        PyErr_Format(PyExc_TypeError, "%s is a torch.dtype, got %s", what, Py_TYPE(o)->tp_name);
         throw PythonError{};
     }
     return reinterpret_cast<THPDtype *>(o)->scalar_type;
@@ -200,7 +203,7 @@ PyObject *layer_forward(PyObject *self, PyObject *const *args, Py_ssize_t n) {
         if (epilogue == -1 && PyErr_Occurred()) throw PythonError{};
         const int64_t M = x.size(0);
         size_t ldy = 0;
-        at::Tensor y = checked_output(l, args[2], M, dtype_arg(args[3], x.scalar_type()), "forward", &ldy);
+        at::Tensor y = checked_output(l, args[2], M, dtype_arg(args[3], x.scalar_type(), "forward: out_dtype"), "forward", &ldy);
         bind_stream(l->ctx, l->device);
         const int xt = act_code(x.scalar_type()), yt = act_code(y.scalar_type());
         const void *xp = x.data_ptr();
@@ -372,6 +375,14 @@ PyObject *quantize_batch(PyObject *, PyObject *const *args, Py_ssize_t n) {
     });
 }
 
+// scales or zero points of a dequantize: f64, on the codes' device, one per group
+at::Tensor group_values(PyObject *o, int device, int64_t groups, const char *what) {
+    const at::Tensor &t = tensor_arg(o, "dequantize_tensor");
+    if (groups > 0 && (!t.is_cuda() || t.get_device() != device || t.scalar_type() != at::kDouble || t.numel() < groups))
+        fail(SHREWQ_ERR_INVALID_ARG, std::string("dequantize_tensor: needs ") + std::to_string(groups) + " float64 " + what + " on the codes' device");
+    return t.is_contiguous() ? t : t.contiguous();
+}
+
 // dequantize(codes, scales, zero points or None, shape, per_channel, dtype) -> tensor
 PyObject *dequantize(PyObject *, PyObject *const *args, Py_ssize_t n) {
     return guarded([&]() -> PyObject * {
@@ -379,11 +390,11 @@ PyObject *dequantize(PyObject *, PyObject *const *args, Py_ssize_t n) {
             PyErr_SetString(PyExc_TypeError, "dequantize(codes, scales, zero_points, shape, per_channel, dtype)");
             throw PythonError{};
         }
-        const at::Tensor &q = tensor_arg(args[0], "dequantize_tensor"), &s = tensor_arg(args[1], "dequantize_tensor");
-        const at::ScalarType type = dtype_arg(args[5], at::kFloat);
+        const at::Tensor &codes = tensor_arg(args[0], "dequantize_tensor");
+        const at::ScalarType type = dtype_arg(args[5], at::kFloat, "dequantize_tensor: the target dtype");
         const int ot = storage_code(type);
         if (ot < 0) fail(SHREWQ_ERR_UNSUPPORTED, "dequantize_tensor: target dtype " + dtype_name(type) + " not supported");
-        const int device = q.get_device();
+        const int device = codes.get_device();
         shrewq_ctx *ctx = context_of(device);
         PyObject *seq = PySequence_Fast(args[3], "dequantize_tensor: shape is a list of sizes");
         if (!seq) throw PythonError{};
@@ -393,11 +404,18 @@ PyObject *dequantize(PyObject *, PyObject *const *args, Py_ssize_t n) {
         if (PyErr_Occurred()) throw PythonError{};
         const Rows rc_ = rows_cols(shape);
         const int gran = (args[4] == Py_True && !shape.empty()) ? SHREWQ_PER_CHANNEL : SHREWQ_PER_TENSOR;
+        const int64_t groups = gran == SHREWQ_PER_CHANNEL ? rc_.rows : 1;
+        // every pointer that a kernel follows, before anything is launched
+        if (!codes.is_cuda() || codes.element_size() != 1 || codes.numel() < rc_.rows * rc_.cols)
+            fail(SHREWQ_ERR_INVALID_ARG, "dequantize_tensor: needs an i8 code for every element of the shape on a CUDA device");
+        const at::Tensor q = codes.is_contiguous() ? codes : codes.contiguous();
+        const at::Tensor s = group_values(args[1], device, rc_.rows * rc_.cols > 0 ? groups : 0, "scales");
+        const at::Tensor z = args[2] == Py_None ? at::Tensor() : group_values(args[2], device, rc_.rows * rc_.cols > 0 ? groups : 0, "zero points");
         at::Tensor out = empty(shape, type, device);
         bind_stream(ctx, device);
         const int8_t *qp = static_cast<const int8_t *>(q.data_ptr());
         const double *sp = static_cast<const double *>(s.data_ptr());
-        const double *zp = args[2] == Py_None ? nullptr : static_cast<const double *>(tensor_arg(args[2], "dequantize_tensor").data_ptr());
+        const double *zp = z.defined() ? static_cast<const double *>(z.data_ptr()) : nullptr;
         void *op = out.data_ptr();
         int rc;
         Py_BEGIN_ALLOW_THREADS
@@ -421,7 +439,6 @@ PyObject *bind(PyObject *, PyObject *args) {
                    {"shrewq_quantize_f32_ex", reinterpret_cast<void **>(&L.quantize_f32_ex)},
                    {"shrewq_quantize_any", reinterpret_cast<void **>(&L.quantize_any)},
                    {"shrewq_quantize_f32_batch", reinterpret_cast<void **>(&L.quantize_f32_batch)},
-                   {"shrewq_dequantize", reinterpret_cast<void **>(&L.dequantize)},
                    {"shrewq_dequantize_ex", reinterpret_cast<void **>(&L.dequantize_ex)},
                    {"shrewq_linear_forward", reinterpret_cast<void **>(&L.linear_forward)},
                    {"shrewq_linear_forward_gate_up_silu", reinterpret_cast<void **>(&L.gate_up_silu)}};
