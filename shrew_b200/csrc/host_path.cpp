@@ -152,10 +152,11 @@ int layer_init(PyObject *self, PyObject *args, PyObject *) {
 
 extern PyTypeObject LayerType;
 
-// x as the library reads it: contiguous, on the layer's device, of a type it takes
-at::Tensor checked_input(const Layer *l, PyObject *o, const char *who) {
+// x as the library reads it: contiguous, on the layer's device, of a type it takes.  any_rank: [M, ..., in_features] of
+// M * in_features elements will do ([M, 1, in_features], say)
+at::Tensor checked_input(const Layer *l, PyObject *o, const char *who, bool any_rank = false) {
     const at::Tensor &x = tensor_arg(o, who);
-    if (x.dim() != 2 || x.size(1) != l->in_features)
+    if (any_rank && x.dim() > 2 ? x.numel() != x.size(0) * l->in_features : x.dim() != 2 || x.size(1) != l->in_features)
         fail(SHREWQ_ERR_INVALID_ARG, std::string(who) + ": expected x of shape [M," + std::to_string(l->in_features) + "], got " + shape_text(x));
     if (act_code(x.scalar_type()) < 0)
         fail(SHREWQ_ERR_UNSUPPORTED, std::string(who) + ": activation dtype " + dtype_name(x.scalar_type()) + " not supported");
@@ -164,7 +165,7 @@ at::Tensor checked_input(const Layer *l, PyObject *o, const char *who) {
 }
 
 // the caller's output buffer, checked, or a new one; its row stride in ldy
-at::Tensor checked_output(const Layer *l, PyObject *out, int64_t M, at::ScalarType type, const char *who, size_t *ldy) {
+at::Tensor checked_output(const Layer *l, PyObject *out, int64_t M, at::ScalarType type, const char *who, size_t *ldy, bool any_rank = false) {
     if (!out || out == Py_None) {
         *ldy = (size_t)l->out_features;
         if (act_code(type) < 0) fail(SHREWQ_ERR_UNSUPPORTED, std::string(who) + ": output dtype " + dtype_name(type) + " not supported");
@@ -175,6 +176,10 @@ at::Tensor checked_output(const Layer *l, PyObject *out, int64_t M, at::ScalarTy
     // (another GPU's memory may be written where the two have peer access)
     if (y.numel() > 0 && (!y.is_cuda() || (y.get_device() != l->device && !at::cuda::get_p2p_access((c10::DeviceIndex)l->device, (c10::DeviceIndex)y.get_device()))))
         fail(SHREWQ_ERR_INVALID_ARG, std::string(who) + ": the output buffer is not on the layer's device");
+    if (any_rank && y.dim() > 2 && y.size(0) == M && y.numel() == M * l->out_features && y.is_contiguous() && act_code(y.scalar_type()) >= 0) {
+        *ldy = (size_t)l->out_features;
+        return y;
+    }
     if (y.dim() != 2 || y.size(0) != M || y.size(1) != l->out_features || (M > 0 && y.stride(1) != 1) || act_code(y.scalar_type()) < 0)
         fail(SHREWQ_ERR_INVALID_ARG, std::string(who) + ": bad output buffer");
     *ldy = (size_t)(M > 1 ? y.stride(0) : std::max(y.stride(0), l->out_features));
@@ -230,10 +235,10 @@ PyObject *layer_gate_up_silu(PyObject *self, PyObject *const *args, Py_ssize_t n
             throw PythonError{};
         }
         const Layer *up = reinterpret_cast<Layer *>(args[0]);
-        const at::Tensor x = checked_input(l, args[1], "gate_up_silu");
+        const at::Tensor x = checked_input(l, args[1], "gate_up_silu", true);
         const int64_t M = x.size(0);
         size_t ldh = 0;
-        at::Tensor y = checked_output(l, args[2], M, x.scalar_type(), "gate_up_silu", &ldh);
+        at::Tensor y = checked_output(l, args[2], M, x.scalar_type(), "gate_up_silu", &ldh, true);
         bind_stream(l->ctx, l->device);
         const int xt = act_code(x.scalar_type()), yt = act_code(y.scalar_type());
         const void *xp = x.data_ptr();

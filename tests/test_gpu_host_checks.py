@@ -47,3 +47,14 @@ def test_dequantize_refuses_what_does_not_cover_the_shape(gran):
     strided = torch.empty(480, dtype=torch.int8, device="cuda")[::2]
     strided.copy_(qt.data)
     assert torch.equal(dequantize_tensor(dataclasses.replace(qt, data=strided)), back)
+
+
+def test_a_gated_pair_takes_rows_of_any_rank():
+    gate, up = _layers()
+    x = torch.randn(5, 1, 128, device="cuda")
+    ref = gate.forward_gate_up_silu(up, x[:, 0])
+    assert torch.equal(gate.forward_gate_up_silu(up, x), ref)
+    out = torch.empty(5, 1, 64, device="cuda")
+    assert gate.forward_gate_up_silu(up, x, out=out) is out and torch.equal(out[:, 0], ref)
+    _refused(lambda: gate.forward_gate_up_silu(up, torch.randn(5, 2, 128, device="cuda")))
+    _refused(lambda: gate.forward(x))       # as ever: forward takes [M, in_features]
