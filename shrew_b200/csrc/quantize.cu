@@ -10,6 +10,8 @@ namespace shrewq {
 
 namespace {
 
+constexpr size_t kMaxGridRows = 0x7FFFFFFF;
+
 template <int GROUP, int NV, typename T, bool ASYM>
 void rows_reg(shrewq_ctx *ctx, const T *w, size_t rows, size_t cols, int8_t *q, double *scales, double *zps, int bits) {
     constexpr int THREADS = GROUP == 32 ? 256 : GROUP;
@@ -83,7 +85,10 @@ int quantize_t(shrewq_ctx *ctx, const T *w, size_t rows, size_t cols, int granul
     *taken = true;
     if (granularity == SHREWQ_PER_CHANNEL) {
         if (rows == 0) return SHREWQ_OK;
-        if (rows > 0x7FFFFFFFull) return set_err(ctx, SHREWQ_ERR_UNSUPPORTED, "quantize: more than 2^31-1 channels");
+        if (rows > kMaxGridRows) {  // a CTA per row or more: left to the kernels whose grid strides over the rows
+            *taken = false;
+            return SHREWQ_OK;
+        }
         *taken = rows_in_registers<T, ASYM>(ctx, w, rows, cols, bits, q, scales, zps);
     } else {
         int rc = tensor_two_pass<T, ASYM>(ctx, w, rows * cols, bits, q, scales, zps);
@@ -95,7 +100,7 @@ int quantize_t(shrewq_ctx *ctx, const T *w, size_t rows, size_t cols, int granul
 
 }  // namespace
 
-// f32, bf16 or f16 tensors in any mode.  *taken false: per-channel rows too long for the register kernels.
+// f32, bf16 or f16 tensors in any mode.  *taken false: per-channel rows too long, or too many, for the register kernels.
 int launch_quantize_tuned(shrewq_ctx *ctx, const void *w, int w_dtype, size_t rows, size_t cols, int granularity, int bits,
                           int mode, int8_t *q, double *scales, double *zps, bool *taken) {
     const bool asym = mode == SHREWQ_ASYMMETRIC;
@@ -112,6 +117,8 @@ int launch_quantize_tuned(shrewq_ctx *ctx, const void *w, int w_dtype, size_t ro
 
 int launch_quantize(shrewq_ctx *ctx, const float *w, size_t rows, size_t cols, int granularity,
                     int8_t *q, double *scales) {
+    if (granularity == SHREWQ_PER_CHANNEL && rows > kMaxGridRows)
+        return set_err(ctx, SHREWQ_ERR_UNSUPPORTED, "quantize: more than 2^31-1 channels");
     bool taken = false;
     int rc = launch_quantize_tuned(ctx, w, SHREWQ_F32, rows, cols, granularity, 8, SHREWQ_SYMMETRIC, q, scales, nullptr, &taken);
     if (rc != SHREWQ_OK || taken) return rc;

@@ -89,3 +89,18 @@ def test_dequantize_in_flat_order(oracle, dtype, gran):
         back = dequantize_tensor(qt).cpu()
         back = back.view(torch.int16).numpy() if dtype is torch.bfloat16 else back.numpy()
         assert back.tobytes() == ref.tobytes(), (rows, cols)
+
+
+def test_more_channels_than_a_grid_has_blocks():
+    # 2^31 rows of one bf16 element: left to the kernel whose grid strides (40 GB in all)
+    from shrew_b200 import quantize_tensor
+    if torch.cuda.mem_get_info()[0] < 60e9:
+        pytest.skip("needs 60 GB free")
+    rows = 1 << 31
+    w = torch.ones((rows, 1), dtype=torch.bfloat16, device="cuda")
+    w[-1] = -3.0
+    qt = quantize_tensor(w, _cfg(8, 0, 1))
+    assert qt.scales.numel() == rows and qt.scales[0].item() == 1.0 / 127.0 and qt.scales[-1].item() == 3.0 / 127.0
+    assert qt.data[-1].item() == -127 and int(qt.data[:-1].min()) == 127
+    del w, qt
+    torch.cuda.empty_cache()
