@@ -90,7 +90,8 @@ SHREWQ_API int shrewq_ctx_set_stream(shrewq_ctx *ctx, void *stream);
  * need no setting.  name / value:
  *   "tc_groups"    1..3   converter groups of the tensor-core kernel (default 3)
  *   "tc_splitk"    0/1    split K when the tile grid leaves SMs idle (default 1)
- *   "tc_tok"       0, 16, 32, 64, 128, 256   force the token tile (default 0 = choose)
+ *   "tc_tok"       0, 16, 32, 64, 128, 256   force the token tile (default 0 = choose); 64 and 128 hold for the persistent
+ *                         f32 kernel too, the CTA-pair kernel always takes 256
  *   "tc_tok_gated" the same for gate/up launches only
  *   "tc_tailsplit" 0..2   a short last wave of tiles as a second launch split along K: 0 (default) = the CTA-pair
  *                         kernel does so for tails of up to a quarter wave, 1 = whenever a tail exists, 2 = never
@@ -106,7 +107,8 @@ SHREWQ_API int shrewq_ctx_set_stream(shrewq_ctx *ctx, void *stream);
  *                         counters only after that kernel has completed (griddepcontrol.wait).  The first forward
  *                         of a handle is always fully ordered behind the stream, so weights quantized on the same
  *                         stream just before are complete; a caller that rewrites a handle's weights in place
- *                         LATER must set 0.  ("gemv_pdl" is accepted as an older name of the same option.)
+ *                         LATER must set 0.  The quantizers launch the same way: they wait for the previous kernel before
+ *                         they touch memory, and the next kernel may start while they run.  ("gemv_pdl" is accepted as an older name of the same option.)
  * Unknown names and values out of range return SHREWQ_ERR_INVALID_ARG. */
 SHREWQ_API int shrewq_ctx_set_option(shrewq_ctx *ctx, const char *name, int value);
 SHREWQ_API int shrewq_ctx_synchronize(shrewq_ctx *ctx);

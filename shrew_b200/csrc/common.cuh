@@ -29,7 +29,7 @@ struct Tuning {
     int tc_pair = 1;        // CTA pairs (tcgen05.mma.cta_group::2) for large batches: 0 never, 1 where they win, 2 whenever M > 128
     int tc_f32 = 1;         // persistent kernel for f32 activations: 0 never, 1 where it wins, 2 whenever it can
     int ring_stages = 0;    // stages of the ring kernel: 0 = by grid size, 2 or 3 forced
-    int pdl = 1;            // programmatic dependent launch of the forward kernels (after a handle's first forward)
+    int pdl = 1;            // programmatic dependent launch of the quantizers and of the forward kernels (after a handle's first forward)
 };
 
 }  // namespace shrewq

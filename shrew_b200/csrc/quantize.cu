@@ -17,14 +17,14 @@ void rows_reg(shrewq_ctx *ctx, const T *w, size_t rows, size_t cols, int8_t *q, 
     constexpr int THREADS = GROUP == 32 ? 256 : GROUP;
     constexpr size_t kRows = GROUP == 32 ? 8 * (8 / NV) : 1;  // rows per CTA
     const size_t grid = (rows + kRows - 1) / kRows;
-    launch_maybe_pdl(quantize_rows_reg_kernel<GROUP, NV, T, ASYM>, dim3((unsigned)grid), dim3(THREADS), 0, ctx->stream, true, w, rows, cols, q, scales, zps,
+    launch_maybe_pdl(quantize_rows_reg_kernel<GROUP, NV, T, ASYM>, dim3((unsigned)grid), dim3(THREADS), 0, ctx->stream, ctx->tuning.pdl != 0, w, rows, cols, q, scales, zps,
                      bits);
 }
 
 template <int GROUP, int NE, typename T, bool ASYM>
 void rows_elem(shrewq_ctx *ctx, const T *w, size_t rows, size_t cols, int8_t *q, double *scales, double *zps, int bits) {
     const unsigned grid = (unsigned)(GROUP == 32 ? (rows + 7) / 8 : rows);
-    launch_maybe_pdl(quantize_rows_elem_kernel<GROUP, NE, T, ASYM>, dim3(grid), dim3(GROUP == 32 ? 256 : GROUP), 0, ctx->stream, true, w, rows, cols, q,
+    launch_maybe_pdl(quantize_rows_elem_kernel<GROUP, NE, T, ASYM>, dim3(grid), dim3(GROUP == 32 ? 256 : GROUP), 0, ctx->stream, ctx->tuning.pdl != 0, w, rows, cols, q,
                      scales, zps, bits);
 }
 
@@ -68,12 +68,12 @@ int tensor_two_pass(shrewq_ctx *ctx, const T *w, size_t n, int bits, int8_t *q, 
     const size_t cap = (size_t)ctx->sm_count * 8 < (size_t)kMaxPartials ? (size_t)ctx->sm_count * 8 : (size_t)kMaxPartials;
     const size_t want = (vecs + 1023) / 1024;
     SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(extrema_partials_kernel<T, ASYM>, dim3((unsigned)(want < 1 ? 1 : (want > cap ? cap : want))), dim3(256), 0,
-                                          ctx->stream, true, w, n, bits, g, scales, zps));
+                                          ctx->stream, ctx->tuning.pdl != 0, w, n, bits, g, scales, zps));
     ctx->launches += 1;
     if (n > 0) {
         constexpr int U = sizeof(T) == 2 ? 2 : 4;
         SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(quantize_tensor_kernel<T, ASYM, U>, dim3((unsigned)(want < 1 ? 1 : (vecs + 256 * U - 1) / (256 * U))),
-                                              dim3(256), 0, ctx->stream, true, w, n, g, q));
+                                              dim3(256), 0, ctx->stream, ctx->tuning.pdl != 0, w, n, g, q));
         ctx->launches += 1;
     }
     return SHREWQ_OK;
@@ -178,10 +178,10 @@ int launch_dequantize(shrewq_ctx *ctx, const int8_t *q, const double *scales, si
     const size_t cap = vec_ok ? 0x7FFFFFFF : (size_t)ctx->sm_count * 32;
     unsigned grid = (unsigned)(want < 1 ? 1 : (want > cap ? cap : want));
     if (out_dtype == SHREWQ_F32)
-        SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(dequantize_kernel<float>, dim3(grid), dim3(256), 0, ctx->stream, true, q, scales, rows, cols, per_channel,
+        SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(dequantize_kernel<float>, dim3(grid), dim3(256), 0, ctx->stream, ctx->tuning.pdl != 0, q, scales, rows, cols, per_channel,
                                               static_cast<float *>(out), vec_ok));
     else
-        SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(dequantize_kernel<uint16_t>, dim3(grid), dim3(256), 0, ctx->stream, true, q, scales, rows, cols, per_channel,
+        SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(dequantize_kernel<uint16_t>, dim3(grid), dim3(256), 0, ctx->stream, ctx->tuning.pdl != 0, q, scales, rows, cols, per_channel,
                                               static_cast<uint16_t *>(out), vec_ok));
     ctx->launches += 1;
     SHREWQ_CUDA_TRY(ctx, cudaGetLastError());

@@ -34,7 +34,7 @@ int launch_quantize_batch(shrewq_ctx *ctx, const shrewq_quant_item *items, size_
         const unsigned grid = (unsigned)(want < 1 ? 1 : (want > cap ? cap : want));
         if (per_channel) {
             if (units > 0) {
-                SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(quantize_batch_rows_kernel, dim3(grid), dim3(kBatchWarps * 32), 0, ctx->stream, true, t));
+                SHREWQ_CUDA_TRY(ctx, launch_maybe_pdl(quantize_batch_rows_kernel, dim3(grid), dim3(kBatchWarps * 32), 0, ctx->stream, ctx->tuning.pdl != 0, t));
                 ctx->launches += 1;
             }
         } else {

@@ -64,3 +64,23 @@ def test_a_per_tensor_quantize_needs_no_workspace_under_capture():
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(q, ref.data) and torch.equal(s, ref.scales)
+
+
+@pytest.mark.parametrize("gran", [0, 1])
+def test_quantizers_under_both_settings_of_dependent_launch(gran):
+    # back to back, each call reading what the one before wrote
+    from shrew_b200 import QuantConfig, dequantize_tensor, quantize_tensor
+    from shrew_b200.quantize import Device, quantize_tensors
+    cfg = QuantConfig.int8_per_channel() if gran else QuantConfig.int8()
+    w = torch.randn((700, 1023), device="cuda")
+    dev, out = Device.get("cuda"), []
+    try:
+        for pdl in (0, 1):
+            dev.set_option("pdl", pdl)
+            qt = quantize_tensor(w, cfg)
+            for _ in range(5):
+                qt = quantize_tensor(dequantize_tensor(qt), cfg)
+            out.append(quantize_tensors([dequantize_tensor(qt)] * 2, cfg)[1])
+    finally:
+        dev.set_option("pdl", 1)
+    assert torch.equal(out[0].data, out[1].data) and torch.equal(out[0].scales, out[1].scales)
