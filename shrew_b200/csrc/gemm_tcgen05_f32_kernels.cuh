@@ -134,7 +134,8 @@ linear_i8_tcgen05_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const f
                 const int n0 = (tile % n_tiles) * kF32Chan;
                 for (int kb = 0; kb < nkb; ++kb, ++it) {
                     const int s = it % C::kWStages;
-                    if (it == C::kWStages) pdl_wait();  // (below)
+                    // the converters free this many stages before they need the first MMA, which needs activations
+                    if (it == C::kWStages + C::kAStages) pdl_wait();
                     if (it >= C::kWStages) ok = f32_wait(bars + C::kWEmpty + 8 * s, ((it / C::kWStages) - 1) & 1, ctl, status, 0, s);
                     if (!ok) break;
                     mbar_expect_tx(bars + C::kWFull + 8 * s, C::kWBytes);
@@ -185,14 +186,13 @@ linear_i8_tcgen05_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const f
         const int total = (end - begin) * nkb;
         for (int it = (warp - 2) >> 2; it < total; it += 2) {
             const int s = it % C::kWStages, as = it % C::kAStages;
-            // as far as the free stages reach the codes are widened while the previous kernel still runs
-            constexpr int kFree = C::kWStages < C::kAStages ? C::kWStages : C::kAStages;
-            if (it == kFree || it == kFree + 1) pdl_wait();
             if (!f32_wait_warp(bars + C::kWFull + 8 * s, (it / C::kWStages) & 1, ctl, status, 4, s)) break;
             uint32_t packed[32];
             convert_row64(smem + C::kWOff + s * C::kWBytes + row * kF32BlockK, swz, packed);
             __syncwarp();
             if (lane == 0) mbar_arrive(bars + C::kWEmpty + 8 * s);
+            // as far as the free operand columns reach the codes are widened while the previous kernel still runs
+            if (it == C::kAStages || it == C::kAStages + 1) pdl_wait();
             if (it >= C::kAStages && !f32_wait_warp(bars + C::kAEmpty + 8 * as, ((it / C::kAStages) - 1) & 1, ctl, status, 5, as)) break;
             tc_fence_after();
             tc_st32(a0 + as * C::kACols, packed);
