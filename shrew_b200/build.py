@@ -8,6 +8,7 @@ travel with the source tree; nothing is written outside the package directory.
 """
 from __future__ import annotations
 
+import importlib.metadata
 import os
 import re
 import subprocess
@@ -83,9 +84,21 @@ def _build(objdir: str, lib: str, flags: list[str], force: bool, verbose: bool) 
 
 def build_host_extension(force: bool = False, verbose: bool = False) -> str:
     """_host.so: csrc/host_path.cpp against the headers and libraries of the installed torch."""
-    src = os.path.join(CSRC, "host_path.cpp")
-    if not force and not _stale(HOST_EXT, _includes(src)):
+    src, stamp = os.path.join(CSRC, "host_path.cpp"), os.path.join(CSRC, "build", "host_extension.txt")
+    against = f"torch {importlib.metadata.version('torch')}, python {sys.version.split()[0]}"   # what a built one matches
+    built = open(stamp).read() if os.path.exists(stamp) else ""
+    if not force and built == against and not _stale(HOST_EXT, _includes(src)):
         return HOST_EXT
+    compile_host_extension(HOST_EXT, verbose=verbose)
+    os.makedirs(os.path.dirname(stamp), exist_ok=True)
+    with open(stamp, "w") as f:
+        f.write(against)
+    return HOST_EXT
+
+
+def compile_host_extension(out: str, flags: list[str] | None = None, verbose: bool = False) -> None:
+    """host_path.cpp with `flags` into the shared object `out` (the CPU tests build one of their own)."""
+    src = os.path.join(CSRC, "host_path.cpp")
     import torch
     root = os.path.dirname(torch.__file__)
     cuda_inc = os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")
@@ -93,14 +106,13 @@ def build_host_extension(force: bool = False, verbose: bool = False) -> str:
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            *[a for d in (os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
                          sysconfig.get_paths()["include"], cuda_inc) for a in ("-isystem", d)],
-           src, "-o", HOST_EXT, "-L" + os.path.join(root, "lib"), "-Wl,-rpath," + os.path.join(root, "lib"),
+           *(flags or []), src, "-o", out, "-L" + os.path.join(root, "lib"), "-Wl,-rpath," + os.path.join(root, "lib"),
            "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or r.returncode != 0:
         sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
     if r.returncode != 0:
         raise RuntimeError("host extension failed to build: " + " ".join(cmd))
-    return HOST_EXT
 
 
 if __name__ == "__main__":

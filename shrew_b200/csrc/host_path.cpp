@@ -8,11 +8,14 @@
 // Nothing is computed here.  Tensors come from torch's caching allocator on torch's current stream, the library is
 // called through addresses that the Python side hands over (bind), so the binding follows whichever build of the
 // library ctypes loaded.  The GIL is released around every library call.
+//
+// The CPU tests build this file with SHREWQ_CPU_EMU: tensors, allocations and device checks are those of the CPU device then.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/cuda/PeerToPeerAccess.h>
+#include <ATen/ops/empty.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/DynamicTypes.h>
 #include <torch/csrc/Dtype.h>
@@ -72,9 +75,23 @@ shrewq_ctx *context_of(int device) {
     return static_cast<shrewq_ctx *>(p);
 }
 
-void bind_stream(shrewq_ctx *ctx, int device) {
-    check(L.set_stream(ctx, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream()), ctx);
+#ifdef SHREWQ_CPU_EMU
+bool on_device(const at::Tensor &t) { return t.device().is_cpu(); }
+int device_index(const at::Tensor &) { return 0; }
+bool peer_access(int, int) { return false; }
+void *current_stream(int) { return nullptr; }
+at::Tensor empty(at::IntArrayRef shape, at::ScalarType t, int) { return at::empty(shape, at::TensorOptions().dtype(t)); }
+#else
+bool on_device(const at::Tensor &t) { return t.is_cuda(); }
+int device_index(const at::Tensor &t) { return (int)t.get_device(); }
+bool peer_access(int from, int to) { return at::cuda::get_p2p_access((c10::DeviceIndex)from, (c10::DeviceIndex)to); }
+void *current_stream(int device) { return c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream(); }
+at::Tensor empty(at::IntArrayRef shape, at::ScalarType t, int device) {
+    return at::Tensor(at::detail::empty_cuda(shape, t, c10::Device(c10::kCUDA, (c10::DeviceIndex)device), std::nullopt));
 }
+#endif
+
+void bind_stream(shrewq_ctx *ctx, int device) { check(L.set_stream(ctx, current_stream(device)), ctx); }
 
 // forward activations and outputs
 int act_code(at::ScalarType t) { return t == at::kFloat ? SHREWQ_F32 : t == at::kBFloat16 ? SHREWQ_BF16 : -1; }
@@ -108,10 +125,6 @@ const at::Tensor &tensor_arg(PyObject *o, const char *who) {
         throw PythonError{};
     }
     return THPVariable_Unpack(o);
-}
-
-at::Tensor empty(at::IntArrayRef shape, at::ScalarType t, int device) {
-    return at::Tensor(at::detail::empty_cuda(shape, t, c10::Device(c10::kCUDA, (c10::DeviceIndex)device), std::nullopt));
 }
 
 PyObject *wrap(at::Tensor t) { return THPVariable_Wrap(std::move(t)); }
@@ -160,7 +173,7 @@ at::Tensor checked_input(const Layer *l, PyObject *o, const char *who, bool any_
         fail(SHREWQ_ERR_INVALID_ARG, std::string(who) + ": expected x of shape [M," + std::to_string(l->in_features) + "], got " + shape_text(x));
     if (act_code(x.scalar_type()) < 0)
         fail(SHREWQ_ERR_UNSUPPORTED, std::string(who) + ": activation dtype " + dtype_name(x.scalar_type()) + " not supported");
-    if (!x.is_cuda() || x.get_device() != l->device) fail(SHREWQ_ERR_INVALID_ARG, std::string(who) + ": x is not on the layer's device");
+    if (!on_device(x) || device_index(x) != l->device) fail(SHREWQ_ERR_INVALID_ARG, std::string(who) + ": x is not on the layer's device");
     return x.is_contiguous() ? x : x.contiguous();
 }
 
@@ -174,7 +187,7 @@ at::Tensor checked_output(const Layer *l, PyObject *out, int64_t M, at::ScalarTy
     }
     const at::Tensor &y = tensor_arg(out, who);
     // (another GPU's memory may be written where the two have peer access)
-    if (y.numel() > 0 && (!y.is_cuda() || (y.get_device() != l->device && !at::cuda::get_p2p_access((c10::DeviceIndex)l->device, (c10::DeviceIndex)y.get_device()))))
+    if (y.numel() > 0 && (!on_device(y) || (device_index(y) != l->device && !peer_access(l->device, device_index(y)))))
         fail(SHREWQ_ERR_INVALID_ARG, std::string(who) + ": the output buffer is not on the layer's device");
     if (any_rank && y.dim() > 2 && y.size(0) == M && y.numel() == M * l->out_features && y.is_contiguous() && act_code(y.scalar_type()) >= 0) {
         *ldy = (size_t)l->out_features;
@@ -291,7 +304,7 @@ PyObject *quantize(PyObject *, PyObject *const *args, Py_ssize_t n) {
         const at::Tensor &t = tensor_arg(args[0], "quantize_tensor");
         const int wt = storage_code(t.scalar_type());
         if (wt < 0) fail(SHREWQ_ERR_UNSUPPORTED, "quantize_tensor: dtype " + dtype_name(t.scalar_type()) + " is not a float storage type");
-        const int device = t.get_device();
+        const int device = device_index(t);
         shrewq_ctx *ctx = context_of(device);
         const at::Tensor w = t.is_contiguous() ? t : t.contiguous();
         const Rows rc_ = rows_cols(w.sizes());
@@ -345,8 +358,8 @@ PyObject *quantize_batch(PyObject *, PyObject *const *args, Py_ssize_t n) {
         int device = -1;
         for (Py_ssize_t i = 0; i < count; ++i) {
             const at::Tensor &t = tensor_arg(PySequence_Fast_GET_ITEM(seq, i), "quantize_tensors");
-            if (i == 0) device = t.get_device();
-            if (t.scalar_type() != at::kFloat || !t.is_cuda() || t.get_device() != device)
+            if (i == 0) device = device_index(t);
+            if (t.scalar_type() != at::kFloat || !on_device(t) || device_index(t) != device)
                 fail(SHREWQ_ERR_UNSUPPORTED, "quantize_tensors: f32 tensors on one CUDA device");
             w.push_back(t.is_contiguous() ? t : t.contiguous());
             const at::Tensor &c = w.back();
@@ -383,7 +396,7 @@ PyObject *quantize_batch(PyObject *, PyObject *const *args, Py_ssize_t n) {
 // scales or zero points of a dequantize: f64, on the codes' device, one per group
 at::Tensor group_values(PyObject *o, int device, int64_t groups, const char *what) {
     const at::Tensor &t = tensor_arg(o, "dequantize_tensor");
-    if (groups > 0 && (!t.is_cuda() || t.get_device() != device || t.scalar_type() != at::kDouble || t.numel() < groups))
+    if (groups > 0 && (!on_device(t) || device_index(t) != device || t.scalar_type() != at::kDouble || t.numel() < groups))
         fail(SHREWQ_ERR_INVALID_ARG, std::string("dequantize_tensor: needs ") + std::to_string(groups) + " float64 " + what + " on the codes' device");
     return t.is_contiguous() ? t : t.contiguous();
 }
@@ -399,7 +412,7 @@ PyObject *dequantize(PyObject *, PyObject *const *args, Py_ssize_t n) {
         const at::ScalarType type = dtype_arg(args[5], at::kFloat, "dequantize_tensor: the target dtype");
         const int ot = storage_code(type);
         if (ot < 0) fail(SHREWQ_ERR_UNSUPPORTED, "dequantize_tensor: target dtype " + dtype_name(type) + " not supported");
-        const int device = codes.get_device();
+        const int device = device_index(codes);
         shrewq_ctx *ctx = context_of(device);
         PyObject *seq = PySequence_Fast(args[3], "dequantize_tensor: shape is a list of sizes");
         if (!seq) throw PythonError{};
@@ -411,7 +424,7 @@ PyObject *dequantize(PyObject *, PyObject *const *args, Py_ssize_t n) {
         const int gran = (args[4] == Py_True && !shape.empty()) ? SHREWQ_PER_CHANNEL : SHREWQ_PER_TENSOR;
         const int64_t groups = gran == SHREWQ_PER_CHANNEL ? rc_.rows : 1;
         // every pointer that a kernel follows, before anything is launched
-        if (!codes.is_cuda() || codes.element_size() != 1 || codes.numel() < rc_.rows * rc_.cols)
+        if (!on_device(codes) || codes.element_size() != 1 || codes.numel() < rc_.rows * rc_.cols)
             fail(SHREWQ_ERR_INVALID_ARG, "dequantize_tensor: needs an i8 code for every element of the shape on a CUDA device");
         const at::Tensor q = codes.is_contiguous() ? codes : codes.contiguous();
         const at::Tensor s = group_values(args[1], device, rc_.rows * rc_.cols > 0 ? groups : 0, "scales");

@@ -1,4 +1,4 @@
-// Launchers of the INT8 symmetric quantize / dequantize kernels (device code and its description:
+// Launchers of the quantize / dequantize kernels (device code and its description:
 // quantize_kernels.cuh).
 #include <cuda_fp16.h>
 
@@ -35,7 +35,7 @@ bool rows_in_registers(shrewq_ctx *ctx, const T *w, size_t rows, size_t cols, in
     const bool vec = cols % EPV == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && (reinterpret_cast<uintptr_t>(q) & (EPV - 1)) == 0;
     const size_t nvec = cols / EPV;
     // Tile widths by the vectors of a row: a warp up to 256 of them, then whole CTAs.  f32 rows of more than 1024 vectors keep
-    // eight per thread (98 % of the copy rate); the 16-bit types, with twice the elements in a vector, keep four.
+    // eight per thread (94 % of the copy rate); the 16-bit types, with twice the elements in a vector, keep four.
     constexpr bool k16 = sizeof(T) == 2;
     if (vec && nvec <= 32) rows_reg<32, 1, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
     else if (vec && nvec <= 64) rows_reg<32, 2, T, ASYM>(ctx, w, rows, cols, q, scales, zps, bits);
@@ -152,9 +152,8 @@ int launch_quantize_given_amax(shrewq_ctx *ctx, const float *w, size_t n, const 
     int rc = ensure_scratch(ctx, 256);
     if (rc != SHREWQ_OK) return rc;
     TensorParams *tp = reinterpret_cast<TensorParams *>(reinterpret_cast<char *>(ctx->scratch) + 64);
-    // n = 1 here: the scale always derives from the supplied amax, also for an empty shard (an
-    // all-empty tensor has amax 0, which gives the same scale 1.0 as the reference's empty case)
-    finalize_tensor_scale_kernel<<<1, 1, 0, ctx->stream>>>(reinterpret_cast<const unsigned int *>(amax_dev), 1, scale, tp);
+    // the scale always derives from the supplied amax, also for an empty shard
+    finalize_tensor_scale_kernel<<<1, 1, 0, ctx->stream>>>(reinterpret_cast<const unsigned int *>(amax_dev), scale, tp);
     ctx->launches += 1;
     if (n > 0) {
         size_t want = (n / 4 + 255) / 256;

@@ -99,7 +99,7 @@ __device__ __forceinline__ void extrema_group(Extrema &e, int t) {
 // 16-byte vectors each.  cols is a multiple of the vector's elements, w is 16-byte and q 4-byte (f32) or 8-byte aligned
 // (checked by the launcher).  Thread 0 forms the f64 parameters while the others already write codes; the undecided
 // elements wait for them at the end (symmetric; an asymmetric row's zero point is needed for every code).
-// 8192 x 8192 f32: 52 us (6.4 TB/s); 66.9 us with two barriers a row, two f64 divisions on the way to the codes and ~20
+// 8192 x 8192 f32: 54 us (6.2 TB/s); 66.9 us with two barriers a row, two f64 divisions on the way to the codes and ~20
 // instructions an element.  (CTAs that walk over rows with the next row's loads in flight were slower: 33 against 29 us
 // for 8192 x 4096, the registers cost more resident rows than the look-ahead gave.)
 template <int GROUP, int NV, typename T = float, bool ASYM = false>
@@ -386,18 +386,11 @@ struct TensorParams {
     RowParams p;
 };
 
-__global__ void finalize_tensor_scale_kernel(const unsigned int *amax_bits, size_t n,
-                                             double *scales, TensorParams *out) {
+// (an empty tensor has amax 0, which gives the reference's scale 1.0 of an empty slice, quantize.rs:340-342)
+__global__ void finalize_tensor_scale_kernel(const unsigned int *amax_bits, double *scales, TensorParams *out) {
     double scale;
     RowParams p;
-    if (n == 0) {  // empty slice: (1.0, 0.0), quantize.rs:340-342
-        scale = 1.0;
-        p.inv64 = 1.0;
-        p.inv32 = 1.0f;
-        p.exact_only = 0;
-    } else {
-        make_params(__uint_as_float(*amax_bits), &scale, &p);
-    }
+    make_params(__uint_as_float(*amax_bits), &scale, &p);
     scales[0] = scale;
     out->p = p;
 }

@@ -27,7 +27,7 @@ int quantize_any_t(shrewq_ctx *ctx, const T *w, size_t rows, size_t cols, int gr
         const unsigned grid = (unsigned)(rows < (size_t)ctx->sm_count * 32 ? rows : (size_t)ctx->sm_count * 32);
         quantize_rows_ex_kernel<T><<<grid, 256, 0, ctx->stream>>>(w, rows, cols, bits, mode, q, scales, zps);
         ctx->launches += 1;
-    } else {
+    } else if constexpr (sizeof(T) == 8) {  // (launch_quantize_tuned takes per-tensor calls of every other type)
         // scratch: [1024, 1024 + sizeof(TensorWords)) of the quantizer's 4 KiB
         int rc = ensure_scratch(ctx, 4096);
         if (rc != SHREWQ_OK) return rc;

@@ -152,9 +152,8 @@ _STORAGE_CODE = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16, torch.float
 # members of the enums above as plain names: class attribute lookups are a noticeable part of a short call
 _INT8, _ASYMMETRIC, _PER_CHANNEL = QuantBits.Int8, QuantMode.Asymmetric, QuantGranularity.PerChannel
 
-# CUDA tensors take the compiled host path (csrc/host_path.cpp): the checks, allocations and library calls of the
-# functions below in one C call each.  The Python statements of the same calls remain for tensors that are not on a
-# CUDA device, whose call ends in Device.get's error.
+# The compiled host path (csrc/host_path.cpp): the checks, allocations and library calls of quantize, dequantize and the
+# forwards in one C call each.  Tensors that are not on a CUDA device end in Device.get's error.
 _host = None
 
 
@@ -198,37 +197,11 @@ def quantize_tensor(tensor: torch.Tensor, config: QuantConfig) -> QuantizedTenso
     """quantize.rs:194-205 on the GPU.  `tensor` is a float CUDA tensor.  f32 INT8 symmetric runs the
     tuned kernels (shrewq_quantize_f32); the other modes and storage types go through
     shrewq_quantize_f32_ex / shrewq_quantize_any."""
-    if tensor.is_cuda:
-        bits, asym = (8 if config.bits is _INT8 else 4), config.mode is _ASYMMETRIC
-        q, scales, zps, shape = (_host or _load_host()).quantize(tensor, config.granularity is _PER_CHANNEL, bits, asym)
-        return QuantizedTensor(q, scales, shape, tensor.dtype, config, zps)
-    dev = Device.get(tensor.device)
-    if tensor.dtype not in _STORAGE_CODE:
-        raise ShrewError(_lib.ERR_UNSUPPORTED, f"quantize_tensor: dtype {tensor.dtype} is not a float storage type")
-    w = tensor.contiguous()
-    shape = list(w.shape)
-    rows, cols = _rows_cols(shape)
-    gran = config.granularity
-    if len(shape) == 0:
-        gran = QuantGranularity.PerTensor
-    n_scales = rows if gran is QuantGranularity.PerChannel else 1
-    q = torch.empty(w.numel(), dtype=torch.int8, device=w.device)
-    scales = torch.empty(n_scales, dtype=torch.float64, device=w.device)
-    dev.bind_stream()
-    if config._is_int8_symmetric() and w.dtype is torch.float32:
-        rc = _lib.lib().shrewq_quantize_f32(dev.handle, _ptr(w), rows, cols, gran.value, _ptr(q), _ptr(scales))
-        _lib.check(rc, dev.handle)
-        return QuantizedTensor(q, scales, shape, tensor.dtype, config)
-    bits, mode = config._abi_mode()
-    zps = torch.empty(n_scales, dtype=torch.float64, device=w.device)
-    if w.dtype is torch.float32:
-        rc = _lib.lib().shrewq_quantize_f32_ex(dev.handle, _ptr(w), rows, cols, gran.value, bits, mode, _ptr(q), _ptr(scales),
-                                               _ptr(zps))
-    else:  # bf16 / f16 / f64 storage: every element is widened to f64 like the reference's to_f64_vec
-        rc = _lib.lib().shrewq_quantize_any(dev.handle, _ptr(w), _STORAGE_CODE[w.dtype], rows, cols, gran.value, bits, mode,
-                                            _ptr(q), _ptr(scales), _ptr(zps))
-    _lib.check(rc, dev.handle)
-    return QuantizedTensor(q, scales, shape, tensor.dtype, config, zps if config.mode is QuantMode.Asymmetric else None)
+    if not tensor.is_cuda:
+        Device.get(tensor.device)    # raises: CUDA devices only
+    bits, asym = (8 if config.bits is _INT8 else 4), config.mode is _ASYMMETRIC
+    q, scales, zps, shape = (_host or _load_host()).quantize(tensor, config.granularity is _PER_CHANNEL, bits, asym)
+    return QuantizedTensor(q, scales, shape, tensor.dtype, config, zps)
 
 
 def quantize_tensors(tensors: Sequence[torch.Tensor], config: QuantConfig) -> List[QuantizedTensor]:
@@ -239,35 +212,10 @@ def quantize_tensors(tensors: Sequence[torch.Tensor], config: QuantConfig) -> Li
         return []
     if not config._is_int8_symmetric():
         raise ShrewError(_lib.ERR_UNSUPPORTED, "quantize_tensors: INT8 symmetric only")
-    if tensors[0].is_cuda:
-        return [QuantizedTensor(q, scales, shape, torch.float32, config) for q, scales, shape in
-                (_host or _load_host()).quantize_batch(tensors, config.granularity is _PER_CHANNEL)]
-    dev = Device.get(tensors[0].device)
-    items = (_lib.QuantItem * len(tensors))()
-    out, keep = [], []
-    per_tensor_group: List[int] = []     # rank-0 tensors fall back to per-tensor (quantize.rs:276-278)
-    for i, t in enumerate(tensors):
-        if t.dtype is not torch.float32 or t.device != tensors[0].device:
-            raise ShrewError(_lib.ERR_UNSUPPORTED, "quantize_tensors: f32 tensors on one CUDA device")
-        w = t.contiguous()
-        shape = list(w.shape)
-        rows, cols = _rows_cols(shape)
-        gran = config.granularity if shape else QuantGranularity.PerTensor
-        if gran is not config.granularity:
-            per_tensor_group.append(i)
-        q = torch.empty(w.numel(), dtype=torch.int8, device=w.device)
-        scales = torch.empty(rows if gran is QuantGranularity.PerChannel else 1, dtype=torch.float64, device=w.device)
-        items[i] = _lib.QuantItem(_ptr(w), rows, cols, _ptr(q), _ptr(scales))
-        keep.append(w)
-        out.append(QuantizedTensor(q, scales, shape, t.dtype, config))
-    dev.bind_stream()
-    main = [i for i in range(len(tensors)) if i not in per_tensor_group]
-    for idx, gran in ((main, config.granularity), (per_tensor_group, QuantGranularity.PerTensor)):
-        if idx:
-            sub = (_lib.QuantItem * len(idx))(*[items[i] for i in idx])
-            _lib.check(_lib.lib().shrewq_quantize_f32_batch(dev.handle, ctypes.cast(sub, ctypes.c_void_p), len(idx), gran.value),
-                       dev.handle)
-    return out
+    if not tensors[0].is_cuda:
+        Device.get(tensors[0].device)
+    return [QuantizedTensor(q, scales, shape, torch.float32, config) for q, scales, shape in
+            (_host or _load_host()).quantize_batch(tensors, config.granularity is _PER_CHANNEL)]
 
 
 def absmax(tensor: torch.Tensor) -> torch.Tensor:
@@ -312,11 +260,12 @@ def pack_int4(qtensor: QuantizedTensor) -> torch.Tensor:
 
 def dequantize_tensor(qtensor: QuantizedTensor, device=None) -> torch.Tensor:
     """quantize.rs:210-225 on the GPU: a tensor of the original dtype and shape."""
-    if device is None and qtensor.data.is_cuda:
+    if device is None:
+        if not qtensor.data.is_cuda:
+            Device.get(qtensor.data.device)
         return (_host or _load_host()).dequantize(qtensor.data, qtensor.scales, qtensor.zero_points_t, qtensor.shape,
                                                   qtensor.config.granularity is _PER_CHANNEL, qtensor.original_dtype)
-    dev_t = qtensor.data.device if device is None else torch.device(device)
-    dev = Device.get(dev_t)
+    dev = Device.get(torch.device(device))
     out_dtype = qtensor.original_dtype
     if out_dtype not in _STORAGE_CODE:
         raise ShrewError(_lib.ERR_UNSUPPORTED, f"dequantize_tensor: target dtype {out_dtype} not supported")

@@ -66,7 +66,7 @@ extern "C" int emu_quantize_tensor(const float *w, size_t n, unsigned grid, int8
     unsigned int *amax_bits = reinterpret_cast<unsigned int *>(scratch);
     TensorParams *tp = reinterpret_cast<TensorParams *>(scratch + 64);
     if (n > 0) emu::launch(grid, 256, [&] { absmax_flat_kernel(w, n, amax_bits); });
-    emu::launch(1, 1, [&] { finalize_tensor_scale_kernel(amax_bits, n, scale, tp); });
+    emu::launch(1, 1, [&] { finalize_tensor_scale_kernel(amax_bits, scale, tp); });
     if (n > 0) emu::launch(grid, 256, [&] { quantize_flat_kernel(w, n, tp, q); });
     return 0;
 }
@@ -75,7 +75,7 @@ extern "C" int emu_quantize_tensor(const float *w, size_t n, unsigned grid, int8
 extern "C" int emu_quantize_given_amax(const float *w, size_t n, const float *amax, unsigned grid, int8_t *q, double *scale) {
     alignas(16) unsigned char scratch[256] = {0};
     TensorParams *tp = reinterpret_cast<TensorParams *>(scratch + 64);
-    emu::launch(1, 1, [&] { finalize_tensor_scale_kernel(reinterpret_cast<const unsigned int *>(amax), 1, scale, tp); });
+    emu::launch(1, 1, [&] { finalize_tensor_scale_kernel(reinterpret_cast<const unsigned int *>(amax), scale, tp); });
     if (n > 0) emu::launch(grid, 256, [&] { quantize_flat_kernel(w, n, tp, q); });
     return 0;
 }
