@@ -89,10 +89,11 @@ quantize_batch_rows_kernel(const BatchTable t) {
     pdl_wait();
     const int lane = threadIdx.x & 31;
     const unsigned int stride = gridDim.x * kBatchWarps * 4u;
-    // (64-bit: up to 2^32 - 1 units, past which the last stride reaches)
-    for (unsigned long long u0 = (blockIdx.x * kBatchWarps + (threadIdx.x >> 5)) * 4u; u0 < t.total_units; u0 += stride) {
-        const unsigned int u_end = u0 + 4u < t.total_units ? (unsigned int)u0 + 4u : t.total_units;
-        unsigned int u = (unsigned int)u0;
+    // (up to 2^32 - 1 units: no sum here may go past the last one)
+    for (unsigned int u0 = (blockIdx.x * kBatchWarps + (threadIdx.x >> 5)) * 4u; u0 < t.total_units;
+         u0 = t.total_units - u0 > stride ? u0 + stride : t.total_units) {
+        const unsigned int u_end = t.total_units - u0 > 4u ? u0 + 4u : t.total_units;
+        unsigned int u = u0;
         while (u < u_end) {
             const BatchItem &it = t.it[batch_find(t, u)];
             const size_t row = u - it.unit_begin, cols = (size_t)it.cols;
