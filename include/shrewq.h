@@ -86,6 +86,11 @@ typedef struct shrewq_linear shrewq_linear;
  * cudaStream_t (NULL = the default stream). */
 SHREWQ_API int shrewq_ctx_create(int device, void *stream, shrewq_ctx **out);
 SHREWQ_API int shrewq_ctx_set_stream(shrewq_ctx *ctx, void *stream);
+/* Streams: calls enqueued on different streams of one context are not ordered among each other.  Quantizing (per channel;
+ * one tensor per tensor, up to eight calls in flight), dequantizing and forwards that are not split along K share nothing.
+ * Forwards split along K, f32 forwards above 1024 features or with bf16 results, layers with zero points, packed INT4
+ * above 4 tokens, batched per-tensor, f64 per-tensor and supplied-amax quantizing and the *_host calls use workspaces of the
+ * context: two of those must not overlap on different streams (order them by events, or use a context per stream). */
 /* Launch options of a context (no counterpart in the reference); the defaults are the measured choices and
  * need no setting.  name / value:
  *   "tc_groups"    1..3   converter groups of the tensor-core kernel (default 3)

@@ -11,21 +11,21 @@
 //  - The grid is what fits the GPU at once and a CTA walks over blocks of 16 rows of W (gated: the gate rows and the up rows
 //    of 8 channels), so that the producer runs on into the next block while this one is multiplied and reduced: gate/up
 //    11008 x 4096 at 8 tokens 29.7 -> 21.1 us, 4096 x 11008 15.9 -> 12.8 us against one block per CTA.  A producer warp asks the copy
-//    engine for them in stages of 16 rows x 512 bytes, one bulk copy per row and stage, into a ring of S stages
-//    (full / empty mbarriers).  With S = 8 a whole K = 4096 row block is requested in the kernel's first hundred
-//    cycles; no load instruction waits in a register scoreboard and the bytes in flight per SM (S * 8 KB per
-//    CTA) do not depend on how many warps are resident.
+//    engine for them in stages of 16 rows x 2 KB, one bulk copy per row and stage, into a ring of two or three stages
+//    (full / empty mbarriers).  Two stages are a whole K = 4096 row block, requested in the kernel's first hundred
+//    cycles; no load instruction waits in a register scoreboard and the bytes in flight per SM (about 200 KB) do not
+//    depend on how many warps are resident.
 //  - Eight consumer warps split every stage by k (four 64-wide k-blocks each).  The weights are the A operand of
 //    mma.sync.m16n8k16 (16 rows x 16 k), the activations the B operand (16 k x 8 tokens): widening a code to
 //    bf16 costs 2.25 instructions whatever the batch (widen_bf16.cuh), and one to four MMAs per step cover 8 to 32 tokens with
 //    the same converted fragment.  Lane (g = lane / 4, t = lane % 4) reads the 16 codes [16t, 16t + 16) of
 //    rows g and g + 8 of the k-block and the 16 activations of the same k for tokens g (+ 8, 16, 24); MMA
 //    step j uses codes and activations 4j .. 4j+3 of those runs for A and B alike (a dot product does not care
-//    about the order of k).  Rows are 576 bytes apart in shared memory, so the 16-byte reads of a quarter warp
+//    about the order of k).  Rows are 2112 bytes apart in shared memory, so the 16-byte reads of a quarter warp
 //    fall into distinct banks.  Activations come straight from global memory (L1 keeps them: every CTA of
-//    an SM reads the same few KB), requested before the wait for the stage.
-//  - The eight warps' accumulators meet in shared memory; 128 (gated: 64) x NT threads apply scale, bias and
-//    the epilogue and store to the local and the peer destinations.
+//    an SM reads the same few KB), requested half a k-block ahead and earlier.
+//  - The eight warps' accumulators meet in shared memory; the 256 consumer threads apply scale, bias and the
+//    epilogue to the 128 (gated: 64) x NT outputs and store to the local and the peer destinations.
 //
 // Programmatic dependent launch: the kernel lets its successor start at once, and its producer requests WEIGHTS
 // without waiting for the predecessor (weights never depend on an earlier kernel); the consumers wait for it
