@@ -1,7 +1,7 @@
 // Weight-only INT8 forward for small batches (M <= 64) on warp-level MMA, sm_100a.
 //
-// The default for 3..32 tokens where the ring kernel (gemv_ring_kernels.cuh) does not win; also the forward of
-// packed INT4 weights.  Its index arithmetic is also checked on the CPU (tests/test_mma_layout.py).
+// The forward of packed INT4 weights, and of INT8 weights by name (shrewq_force_kernel): by default the ring kernel
+// (gemv_ring_kernels.cuh) runs 3..32 tokens, above 16 with the same sums.  Its index arithmetic is also checked on the CPU (tests/test_mma_layout.py).
 //
 // Why it exists: for 4 < M <= 64 the layer is HBM-bound, but the tcgen05 kernel feeds the
 // tensor core from ONE issuing thread per CTA (about 80 cycles per instruction, each covering

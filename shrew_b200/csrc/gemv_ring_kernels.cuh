@@ -32,8 +32,8 @@
 // before they read activations or write outputs.  A chain of small-batch forwards thus keeps the weight stream
 // going across kernel boundaries.  Launched without the attribute the two instructions do nothing.
 //
-// Every wait is bounded, and none that depends on the consumers starts before the previous kernel has completed: a wait that runs out records itself in DeviceStatus (timeout code 4) and the CTA
-// leaves without writing.
+// Every wait is bounded, and none that depends on the consumers starts before the previous kernel has completed.  A wait that
+// runs out records itself in DeviceStatus (timeout code 4) and the CTA leaves without writing.
 //
 // Device code only (PTX behind ptx_small.cuh / ptx_tcgen05.cuh): also compiles against the CUDA stand-in of the
 // CPU tests (tests/cpu_emu/).
